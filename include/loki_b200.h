@@ -366,7 +366,8 @@ int lk_sweep_results(const lk_sweep* sw, double* params, float* scores, uint64_t
 /* Launch-shape tuning (an autotuner of this library; no reference counterpart).
  * bf_*: brute fold rows (E, V) per consumer warp (1 or 2), consumer warps
  * per block (0: the wave-count rule), shared-memory ring depth in 32-sample
- * words; merge_rows_in_flight: output rows per warp whose loads are issued
+ * words (32: the run form, whose depth follows from the memory its sums leave);
+ * merge_rows_in_flight: output rows per warp whose loads are issued
  * together in a merge level (0: the default for nbins); score_cells_per_block:
  * final cells per block of the fused final level (0: the most that fit). */
 typedef struct lk_tuning {
@@ -436,6 +437,13 @@ void lk_brute_fold_destroy(lk_brute_fold* bf);
 /* d_fold: [nsamps/segment_len, nfreqs, 2, nbins] FP32. */
 int lk_brute_fold_execute(lk_brute_fold* bf, const float* d_ts_e, const float* d_ts_v,
                           float* d_fold, lk_stream_t stream);
+/* Host replay (no device) of the run tables of the brute fold's run form
+ * over one segment `ts` [segment_len] of one row, every read checked against
+ * the padded segment: fold [nfreqs * nbins]; *applies = 0 (fold untouched)
+ * where that form does not take these frequencies. */
+int lk_brute_fold_replay(const double* freqs, uint64_t nfreqs, uint64_t segment_len,
+                         uint64_t nbins, double tsamp, double t_ref, const float* ts, float* fold,
+                         int* applies);
 
 /* ---- boxcar S/N -------------------------------------------------------- */
 /* detection::generate_box_width_trials (lib/score.cpp:390-405): writes up to

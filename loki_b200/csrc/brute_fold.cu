@@ -51,12 +51,12 @@
 #include <cstring>
 #include <numeric>
 #include <string>
-#include <thread>
 #include <type_traits>
 
 #include <cudaTypedefs.h>
 
 #include "lk_device.cuh"
+#include "lk_fold_runs.hpp"
 #include "lk_kernels.hpp"
 #include "lk_ptx.cuh"
 
@@ -66,6 +66,7 @@ namespace {
 
 constexpr int kWarp = 32;
 constexpr int kMaxStages = 16;
+constexpr uint32_t kDefaultStages = 3;
 constexpr uint32_t kTileBytes = 32 * 32 * sizeof(float);  // 32 samples x 32 segments
 constexpr uint32_t kStageBytes = 2 * kTileBytes;           // E and V rows, 8 KiB
 constexpr size_t kSmemLimit = 227 * 1024;
@@ -1065,6 +1066,51 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
+// The sample -> bin map is non-decreasing (mod nbins) in the sample index: every
+// operation of host_phase_bin is monotone in it. With at least two samples per
+// bin a run's end is therefore found from its expected place by stepping to the
+// sample where the bin changes, two evaluations a run instead of one a sample.
+std::vector<FoldRuns> fold_runs(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
+                                double tsamp, double t_ref) {
+    std::vector<FoldRuns> per_f(freqs.size());
+    parallel_for(freqs.size(), segment_len / 8, [&](uint64_t f) {
+        const double freq = freqs[f];
+        auto bin = [&](uint64_t i) {
+            return host_phase_bin((static_cast<double>(i) * tsamp) - t_ref, freq, nbins);
+        };
+        auto& rb = per_f[f];
+        const double step = freq * tsamp * static_cast<double>(nbins);  // bins per sample
+        const bool jump = step < 0.5;
+        double edge = 0.0;  // expected end of the current run, in samples
+        if (jump && step > 0.0) {
+            const double phase = -t_ref * freq;
+            const double at = (phase - std::floor(phase)) * static_cast<double>(nbins) + 0.5;
+            edge = (1.0 - (at - std::floor(at))) / step;
+            rb.start.reserve(static_cast<size_t>(static_cast<double>(segment_len) * step) + 8);
+            rb.bin.reserve(rb.start.capacity());
+        }
+        for (uint64_t i = 0; i < segment_len;) {
+            const uint32_t b = bin(i);
+            rb.start.push_back(static_cast<uint32_t>(i));
+            rb.bin.push_back(static_cast<uint16_t>(b));
+            uint64_t j = i + 1;
+            if (jump) {
+                const double g = step > 0.0 ? std::ceil(edge) : static_cast<double>(segment_len);
+                j = g > static_cast<double>(segment_len) ? segment_len : std::max(j, static_cast<uint64_t>(g));
+                while (j > i + 1 && bin(j - 1) != b) {
+                    --j;
+                }
+                edge += step > 0.0 ? 1.0 / step : 0.0;
+            }
+            while (j < segment_len && bin(j) == b) {
+                ++j;
+            }
+            i = j;
+        }
+    });
+    return per_f;
+}
+
 BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segment_len,
                                  uint64_t nbins, uint64_t nsamps, double tsamp, double t_ref,
                                  uint32_t* d_status)
@@ -1072,6 +1118,9 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
       m_seglen(segment_len),
       m_nbins(nbins),
       m_nsamps(nsamps),
+      m_freqs(freqs),
+      m_tsamp(tsamp),
+      m_t_ref(t_ref),
       m_status(d_status) {
     require(!freqs.empty(), "BruteFold: Frequency array is empty");
     require(segment_len > 0 && nsamps % segment_len == 0,
@@ -1098,7 +1147,7 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     // 2 .. 16 words on the 2^22-sample accelerated workload changed nothing
     // but the shared memory left for accumulators), so 3 words leave the
     // most for accumulator warps. LOKI_B200_BF_STAGES overrides it (2 .. 16).
-    uint32_t stages = 3;
+    uint32_t stages = kDefaultStages;
     if (const char* env = std::getenv("LOKI_B200_BF_STAGES")) {
         stages = std::max<uint32_t>(2, std::min<uint32_t>(kMaxStages, std::atoi(env)));
     }
@@ -1114,45 +1163,40 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     }
     require(configure(rows, warps, stages),
             "BruteFold: nbins too large for the shared-memory accumulators");
+    m_runs = std::make_unique<RunFold>(fold_runs(freqs, segment_len, nbins, tsamp, t_ref), m_seglen, m_nbins);
+    if (!m_runs->ok()) {
+        m_runs.reset();
+    } else if (std::getenv("LOKI_B200_BF_ROWS") == nullptr && std::getenv("LOKI_B200_BF_WARPS") == nullptr &&
+               std::getenv("LOKI_B200_BF_STAGES") == nullptr) {
+        configure(2, 0, run_form_stages());
+    }
+    m_ready = true;
+    if (!m_use_runs) {
+        make_tables();
+    }
+}
 
+// Tables of the forms that walk samples (made when one of them is selected).
+void BruteFoldDevice::make_tables() {
+    if (!m_ready || m_masks.ptr != nullptr) {
+        return;
+    }
     // Run tables, one frequency per task (host threads; same arithmetic as
     // the reference's BruteFold::compute_phase_time_domain, lib/fold.cpp:113-142).
+    const std::vector<FoldRuns> per_f = fold_runs(m_freqs, m_seglen, m_nbins, m_tsamp, m_t_ref);
     std::vector<uint32_t> masks(m_nfreq * m_nwords, 0u);
-    std::vector<std::vector<uint16_t>> per_f(m_nfreq);
-    const unsigned nthreads =
-        std::max(1u, std::min<unsigned>(std::thread::hardware_concurrency(), 32u));
-    auto work = [&](unsigned tid) {
-        for (uint64_t f = tid; f < m_nfreq; f += nthreads) {
-            uint32_t* mw = masks.data() + f * m_nwords;
-            auto& rb = per_f[f];
-            uint32_t prev = 0xffffffffu;
-            for (uint64_t i = 0; i < segment_len; ++i) {
-                const double proper_time = (static_cast<double>(i) * tsamp) - t_ref;
-                const uint32_t b = host_phase_bin(proper_time, freqs[f], nbins);
-                if (b != prev) {
-                    mw[i / 32] |= 1u << (i % 32);
-                    rb.push_back(static_cast<uint16_t>(b));
-                    prev = b;
-                }
-            }
-        }
-    };
-    {
-        std::vector<std::thread> pool;
-        for (unsigned t = 0; t < nthreads; ++t) {
-            pool.emplace_back(work, t);
-        }
-        for (auto& t : pool) {
-            t.join();
+    for (uint64_t f = 0; f < m_nfreq; ++f) {
+        for (const uint32_t i : per_f[f].start) {
+            masks[f * m_nwords + i / 32] |= 1u << (i % 32);
         }
     }
     // Frequencies whose run bins step by one bin (mod nbins) at every run.
     std::vector<uint8_t> seq(m_nfreq, 0);
     for (uint64_t f = 0; f < m_nfreq; ++f) {
-        const auto& rb = per_f[f];
+        const auto& rb = per_f[f].bin;
         bool ok = !rb.empty();
         for (size_t k = 1; ok && k < rb.size(); ++k) {
-            ok = rb[k] == (rb[k - 1] + 1) % nbins;
+            ok = rb[k] == (rb[k - 1] + 1) % m_nbins;
         }
         seq[f] = ok ? 1 : 0;
     }
@@ -1160,17 +1204,17 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     uint64_t total = 0;
     for (uint64_t f = 0; f < m_nfreq; ++f) {
         off[f] = total;
-        nruns[f] = per_f[f].size();
-        total += per_f[f].size();
+        nruns[f] = per_f[f].bin.size();
+        total += per_f[f].bin.size();
     }
     const size_t bsz = m_wide_bins ? 2 : 1;
     std::vector<unsigned char> bins(std::max<uint64_t>(total, 1) * bsz);
     for (uint64_t f = 0; f < m_nfreq; ++f) {
-        for (uint64_t k = 0; k < per_f[f].size(); ++k) {
+        for (uint64_t k = 0; k < per_f[f].bin.size(); ++k) {
             if (m_wide_bins) {
-                std::memcpy(bins.data() + (off[f] + k) * 2, &per_f[f][k], 2);
+                std::memcpy(bins.data() + (off[f] + k) * 2, &per_f[f].bin[k], 2);
             } else {
-                bins[off[f] + k] = static_cast<unsigned char>(per_f[f][k]);
+                bins[off[f] + k] = static_cast<unsigned char>(per_f[f].bin[k]);
             }
         }
     }
@@ -1184,8 +1228,13 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     LK_CUDA(cudaMemcpy(m_nruns.ptr, nruns.data(), m_nruns.bytes, cudaMemcpyHostToDevice));
     m_seq.alloc(m_nfreq);
     LK_CUDA(cudaMemcpy(m_seq.ptr, seq.data(), m_nfreq, cudaMemcpyHostToDevice));
-    m_nseq = static_cast<uint64_t>(std::count(seq.begin(), seq.end(), uint8_t{1}));
 }
+
+BruteFoldDevice::~BruteFoldDevice() = default;
+
+bool BruteFoldDevice::has_run_form() const { return m_runs != nullptr; }
+uint32_t BruteFoldDevice::run_form_stages() { return RunFold::marker_stages(); }
+uint32_t BruteFoldDevice::max_run_form_warps() const { return m_runs ? m_runs->max_warps() : 0; }
 
 // Launch shape: rows (E, V) per consumer warp, consumer warps per block
 // (0: the fewest waves of blocks over the SMs among W >= 3/4 of the most that
@@ -1204,6 +1253,23 @@ uint32_t BruteFoldDevice::max_tmem_warps(uint32_t smem_warps) const {
 }
 
 bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem) {
+    if (rows == 2 && tmem == 0 && stages == run_form_stages() && m_runs) {
+        const uint32_t w = warps != 0 ? warps : m_runs->default_warps(m_nseg);
+        if (w == 0 || w > m_runs->max_warps() || m_runs->blocks_per_group(w) > 65535) {
+            return false;
+        }
+        m_rows = rows;
+        m_warps = w;
+        m_stages = stages;
+        m_tmem = 0;
+        m_use_runs = true;
+        m_map_e_ptr = nullptr;
+        m_map_ev_ptr = nullptr;
+        return true;
+    }
+    if (stages == run_form_stages()) {
+        stages = kDefaultStages;  // a run-form depth with another form's rows or TMEM warps
+    }
     if ((rows != 1 && rows != 2) || stages < 2 || stages > kMaxStages) {
         return false;
     }
@@ -1225,6 +1291,8 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
         // at least half the SM's shared memory: one block per SM, so a
         // second block never waits for the first one's tensor memory
         m_smem = std::max<size_t>(smem, 116 * 1024);
+        m_use_runs = false;
+        make_tables();
         m_map_e_ptr = nullptr;
         m_map_ev_ptr = nullptr;
         return true;
@@ -1259,6 +1327,8 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
     m_stages = stages;
     m_tmem = 0;
     m_smem = ring + w * per_warp;
+    m_use_runs = false;
+    make_tables();
     m_map_e_ptr = nullptr;  // the input binding depends on the rows
     m_map_ev_ptr = nullptr;
     return true;
@@ -1275,7 +1345,7 @@ uint32_t BruteFoldDevice::max_warps(uint32_t rows, uint32_t stages) const {
 
 uint64_t BruteFoldDevice::device_bytes() const {
     return m_masks.bytes + m_bins.bytes + m_bin_off.bytes + m_nruns.bytes + m_stage.bytes +
-           m_ev.bytes + m_seq.bytes + m_groups.bytes;
+           m_ev.bytes + m_seq.bytes + m_groups.bytes + (m_runs ? m_runs->device_bytes() : 0);
 }
 
 // The TMA maps read the series in place; a base address that is not 16-byte
@@ -1283,9 +1353,18 @@ uint64_t BruteFoldDevice::device_bytes() const {
 // A batch of nbatch series stored back to back is folded as one series of
 // nbatch * nseg segments: every segment is folded from its own start.
 void BruteFoldDevice::bind_inputs(const float* d_ts_e, const float* d_ts_v, cudaStream_t s,
-                                  uint64_t nbatch) {
+                                  uint64_t nbatch, const uint64_t* d_lens) {
     require(nbatch >= 1, "BruteFold: nbatch must be positive");
     const uint64_t n = nbatch * m_nsamps;
+    if (m_use_runs) {
+        require(nbatch * m_nseg <= 0x7fffffffULL, "BruteFold: too many segments");
+        m_bound_groups = make_groups(d_lens, nbatch, s);
+        const uint32_t* tab = m_bound_groups ? m_groups.as<uint32_t>() : nullptr;
+        m_runs->transpose(d_ts_e, d_ts_v, nbatch * m_nseg, tab ? tab + 1 + nbatch : nullptr, tab, s);
+        m_map_batch = nbatch;
+        m_map_e_ptr = d_ts_e;  // marks the inputs as bound
+        return;
+    }
     if (m_rows == 2) {
         if (m_ev.bytes < n * sizeof(float2)) {
             m_ev.alloc(n * sizeof(float2));
@@ -1358,20 +1437,24 @@ void BruteFoldDevice::fold(float* d_fold, cudaStream_t s, const uint64_t* d_lens
     // Group mode: only the segments that hold samples are folded (in groups
     // of 8); the grid keeps its full size so that a captured graph stays
     // valid for any lengths, and blocks past the groups return at once.
-    const bool grouped = d_lens != nullptr && m_rows == 2 && m_nseg % 8 == 0;
+    const bool grouped = m_use_runs ? m_bound_groups : make_groups(d_lens, m_map_batch, s);
     if (grouped) {
-        const uint64_t ngmax = nseg / 8;
-        const uint64_t words = 1 + m_map_batch + ngmax;
-        if (m_groups.bytes < words * sizeof(uint32_t)) {
-            m_groups.alloc(words * sizeof(uint32_t));
-        }
         uint32_t* tab = m_groups.as<uint32_t>();
-        seg_groups_kernel<<<1, 256, 0, s>>>(d_lens, static_cast<uint32_t>(m_map_batch),
-                                            static_cast<uint32_t>(m_nseg), m_seglen, tab);
-        LK_CUDA(cudaGetLastError());
         a.ngroups = tab;
         a.groups = tab + 1 + m_map_batch;
-        grid.x = static_cast<unsigned>((ngmax + 3) / 4);
+        grid.x = static_cast<unsigned>((nseg / 8 + 3) / 4);
+    }
+    auto zero_skipped = [&] {
+        if (grouped) {
+            zero_skipped_kernel<<<static_cast<unsigned>(nseg), 256, 0, s>>>(
+                d_lens, static_cast<uint32_t>(m_nseg), m_seglen, m_nfreq * 2 * m_nbins, d_fold);
+            LK_CUDA(cudaGetLastError());
+        }
+    };
+    if (m_use_runs) {
+        m_runs->fold(d_fold, nseg, m_warps, a.groups, a.ngroups, m_status, s);
+        zero_skipped();
+        return;
     }
     auto launch = [&](auto kern) {
         LK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1397,11 +1480,23 @@ void BruteFoldDevice::fold(float* d_fold, cudaStream_t s, const uint64_t* d_lens
                     : launch(brute_fold_mask_kernel<uint8_t, 1>);
     }
     LK_CUDA(cudaGetLastError());
-    if (grouped) {
-        zero_skipped_kernel<<<static_cast<unsigned>(nseg), 256, 0, s>>>(
-            d_lens, static_cast<uint32_t>(m_nseg), m_seglen, m_nfreq * 2 * m_nbins, d_fold);
-        LK_CUDA(cudaGetLastError());
+    zero_skipped();
+}
+
+// Segment-group table of a batch whose series hold d_lens samples each (two
+// rows per warp and nseg a multiple of 8; otherwise every segment is folded).
+bool BruteFoldDevice::make_groups(const uint64_t* d_lens, uint64_t nbatch, cudaStream_t s) {
+    if (d_lens == nullptr || m_rows != 2 || m_nseg % 8 != 0) {
+        return false;
     }
+    const uint64_t words = 1 + nbatch + nbatch * m_nseg / 8;
+    if (m_groups.bytes < words * sizeof(uint32_t)) {
+        m_groups.alloc(words * sizeof(uint32_t));
+    }
+    seg_groups_kernel<<<1, 256, 0, s>>>(d_lens, static_cast<uint32_t>(nbatch), static_cast<uint32_t>(m_nseg),
+                                        m_seglen, m_groups.as<uint32_t>());
+    LK_CUDA(cudaGetLastError());
+    return true;
 }
 
 }  // namespace lk

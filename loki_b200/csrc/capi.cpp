@@ -11,6 +11,7 @@
 #include "lk_device.cuh"
 #include "lk_dts.hpp"
 #include "lk_ffa.hpp"
+#include "lk_fold_runs.hpp"
 #include "lk_fourier.hpp"
 #include "lk_kernels.hpp"
 #include "lk_mc.hpp"
@@ -745,6 +746,20 @@ void lk_brute_fold_destroy(lk_brute_fold* bf) {
             delete bf;
         }
     }
+}
+
+int lk_brute_fold_replay(const double* freqs, uint64_t nfreqs, uint64_t segment_len,
+                         uint64_t nbins, double tsamp, double t_ref, const float* ts, float* fold,
+                         int* applies) {
+    return guarded([&] {
+        need(freqs, "freqs");
+        need(ts, "ts");
+        need(fold, "fold");
+        need(applies, "applies");
+        lk::require(segment_len > 0 && nbins >= 1 && nbins <= 65535, "BruteFold: bad segment length or nbins");
+        const auto runs = lk::fold_runs(std::vector<double>(freqs, freqs + nfreqs), segment_len, nbins, tsamp, t_ref);
+        *applies = lk::run_fold_replay(runs, segment_len, nbins, ts, fold) ? 1 : 0;
+    });
 }
 
 int lk_brute_fold_execute(lk_brute_fold* bf, const float* d_ts_e, const float* d_ts_v,

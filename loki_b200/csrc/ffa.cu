@@ -170,10 +170,10 @@ const void* FFAExec::run_levels(const float* ts_e, const float* ts_v, uint32_t l
     if (bf->interleaves()) {
         // (e, v) pairs for the packed brute fold: series in, pairs out
         prof.begin(LK_STAGE_INTERLEAVE, 0, 1, 2 * series_bytes, s);
-        bf->bind_inputs(ts_e, ts_v, s, nbatch);
+        bf->bind_inputs(ts_e, ts_v, s, nbatch, batch_lens);
         prof.end(s);
     } else {
-        bf->bind_inputs(ts_e, ts_v, s, nbatch);
+        bf->bind_inputs(ts_e, ts_v, s, nbatch, batch_lens);
     }
     prof.begin(LK_STAGE_BRUTE_FOLD, 0, 1, series_bytes + 4 * plan.fold_size(0) * nbatch, s);
     bf->fold(static_cast<float*>(in), s, batch_lens);
@@ -399,7 +399,22 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
         // best packed (two-row) shared-memory shape, the base of step 1b
         float pk_best = INFINITY;
         uint32_t pw = 0, ps = stages0;
-        for (uint32_t rows = 1; rows <= 2; ++rows) {
+        // The run form was faster than every shape of the other forms at each
+        // size tried, so where the plan has it only its warps are tuned.
+        const bool runs = bf->has_run_form();
+        for (uint32_t w = runs ? bf->max_run_form_warps() : 0; w >= 4; --w) {
+            if (!bf->configure(2, w, BruteFoldDevice::run_form_stages())) {
+                continue;
+            }
+            const float ms = time_stages({LK_STAGE_INTERLEAVE, LK_STAGE_BRUTE_FOLD});
+            if (ms < bf_best) {
+                bf_best = ms;
+                br = 2;
+                bw = w;
+                bs = bf->stages();
+            }
+        }
+        for (uint32_t rows = runs ? 3 : 1; rows <= 2; ++rows) {
             if (rows == 2 && plan.cfg.nbins > 128) {
                 continue;
             }

@@ -1,0 +1,90 @@
+// Run form of the brute fold (brute_fold_runs.cu): host tables and launch.
+#pragma once
+
+#include <algorithm>
+#include <atomic>
+#include <cstdint>
+#include <thread>
+#include <vector>
+
+#include "lk_kernels.hpp"
+
+namespace lk {
+
+// The runs of one trial frequency over one segment, in sample order: the first
+// sample and the bin of each run of equal bin.
+struct FoldRuns {
+    std::vector<uint32_t> start;
+    std::vector<uint16_t> bin;
+};
+
+// fn(i) for i < n on host threads: about one per 2^16 units of work (`each` per
+// item), at most 32.
+template <class F>
+void parallel_for(uint64_t n, uint64_t each, F&& fn) {
+    const uint64_t want = n * (each + 1) / 65536 + 1;
+    const auto nthreads = static_cast<unsigned>(
+        std::min<uint64_t>({want, n, 32, std::max(1u, std::thread::hardware_concurrency())}));
+    std::atomic<uint64_t> next{0};
+    auto work = [&] {
+        for (uint64_t i = next++; i < n; i = next++) {
+            fn(i);
+        }
+    };
+    std::vector<std::thread> pool;
+    for (unsigned t = 1; t < nthreads; ++t) {
+        pool.emplace_back(work);
+    }
+    work();
+    for (auto& t : pool) {
+        t.join();
+    }
+}
+
+// Host replay of the run form's tables over one segment of one row (fold:
+// [nfreq][nbins]), with the kernel's reads checked against the padded segment;
+// false where the form does not apply.
+bool run_fold_replay(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, const float* ts,
+                     float* fold);
+
+// Run table of every frequency (host threads).
+std::vector<FoldRuns> fold_runs(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
+                                double tsamp, double t_ref);
+
+class RunFold {
+public:
+    // Builds the tables; ok() is false when a frequency's runs do not have
+    // the form the kernel takes (see brute_fold_runs.cu).
+    RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins);
+    bool ok() const { return m_ok; }
+    // Consumer warps per block the kernel allows, and the default for a fold
+    // of nseg segments.
+    uint32_t max_warps() const;
+    uint32_t default_warps(uint64_t nseg) const;
+    uint64_t blocks_per_group(uint32_t warps) const {
+        return static_cast<uint64_t>(m_nranges) * ((m_nfreq + warps - 1) / warps);
+    }
+    // Ring depth that names this form in a launch shape (its real depth
+    // follows from the shared memory the sums leave).
+    static uint32_t marker_stages();
+    // Transposes nrows segments into [group of 32][sample][32 lanes] (e, v)
+    // pairs. groups / ngroups: the segment-group table (nullptr: all rows in
+    // order).
+    void transpose(const float* d_e, const float* d_v, uint64_t nrows, const uint32_t* groups,
+                   const uint32_t* ngroups, cudaStream_t s);
+    void fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t* groups,
+              const uint32_t* ngroups, uint32_t* d_status, cudaStream_t s) const;
+    uint64_t device_bytes() const { return m_items.bytes + m_rots.bytes + m_bits.bytes + m_evt.bytes; }
+
+private:
+    bool m_ok = false;
+    uint32_t m_nfreq, m_nbins, m_seglen;
+    uint32_t m_nranges = 1, m_range = 0;  // bin ranges per frequency, bins per range
+    uint32_t m_pad = 0;                   // zero samples before each segment
+    uint32_t m_nstages = 0;               // stages of one padded segment
+    DeviceBuffer m_items, m_rots, m_bits, m_evt;
+    uint32_t m_wpr = 1;
+    uint64_t m_evt_groups = 0;
+};
+
+}  // namespace lk

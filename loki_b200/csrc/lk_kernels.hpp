@@ -46,10 +46,12 @@ struct DeviceBuffer {
 // 32 samples plus the bin of each run. Replaying the runs in order adds every
 // sample to its bin in increasing sample order, which is the reference's
 // summation order (lib/kernels.cpp:550-580), so the fold is bit-identical.
+class RunFold;
 class BruteFoldDevice {
 public:
     BruteFoldDevice(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
                     uint64_t nsamps, double tsamp, double t_ref, uint32_t* d_status);
+    ~BruteFoldDevice();
     // Enqueue the fold of (d_ts_e, d_ts_v); d_fold must hold nseg * nfreq * 2 *
     // nbins floats.
     void execute(const float* d_ts_e, const float* d_ts_v, float* d_fold, cudaStream_t s) {
@@ -59,20 +61,25 @@ public:
     // Points the input tensor maps at the series, or at nbatch series of
     // nsamps samples stored back to back. fold() then folds all of them:
     // d_fold holds nbatch * fold_size() floats. With both rows per warp the
-    // series are first interleaved into (e, v) pairs on `s` (one kernel);
-    // otherwise the maps read them in place (a misaligned series is first
-    // copied into an aligned buffer on `s`).
+    // series are first interleaved into (e, v) pairs on `s` (one kernel; the
+    // run form's transposition skips the segments past d_lens, see
+    // fold()); otherwise the maps read them in place (a misaligned series is
+    // first copied into an aligned buffer on `s`).
     void bind_inputs(const float* d_ts_e, const float* d_ts_v, cudaStream_t s,
-                     uint64_t nbatch = 1);
+                     uint64_t nbatch = 1, const uint64_t* d_lens = nullptr);
     // True when bind_inputs launches the interleave kernel.
     bool interleaves() const { return m_rows == 2; }
     // Launch shape (see brute_fold.cu); false when it does not fit. tmem:
     // consumer warps (of `warps`) whose sums live in tensor memory (packed
-    // form only).
+    // form only). Two rows and stages == run_form_stages() select the
+    // run form (brute_fold_runs.cu), the default where it applies.
     bool configure(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem = 0);
     uint32_t max_warps(uint32_t rows, uint32_t stages) const;
     // Most tensor-memory warps a block of smem_warps shared-memory warps can add.
     uint32_t max_tmem_warps(uint32_t smem_warps) const;
+    bool has_run_form() const;
+    static uint32_t run_form_stages();
+    uint32_t max_run_form_warps() const;
     uint32_t rows() const { return m_rows; }
     uint32_t warps() const { return m_warps; }
     uint32_t stages() const { return m_stages; }
@@ -89,7 +96,14 @@ public:
     uint64_t device_bytes() const;
 
 private:
+    // Builds the segment-group table of the bound batch on s when d_lens
+    // applies (see fold()); returns whether it does.
+    bool make_groups(const uint64_t* d_lens, uint64_t nbatch, cudaStream_t s);
+    void make_tables();
     uint64_t m_nfreq, m_seglen, m_nbins, m_nsamps, m_nseg = 0;
+    std::vector<double> m_freqs;
+    double m_tsamp, m_t_ref;
+    bool m_ready = false;      // the form has been chosen
     uint64_t m_nwords = 0;
     bool m_wide_bins = false;  // uint16 run bins (nbins > 256)
     uint32_t m_rows = 2;       // rows (E, V) per consumer warp
@@ -103,7 +117,6 @@ private:
     DeviceBuffer m_bin_off;    // uint64 first run of each frequency
     DeviceBuffer m_nruns;      // uint64 runs of each frequency
     DeviceBuffer m_seq;        // uint8 per frequency: run bins step by one
-    uint64_t m_nseq = 0;
     DeviceBuffer m_stage;      // aligned copy of a misaligned series
     DeviceBuffer m_ev;         // (e, v) interleaved series (both rows per warp)
     CUtensorMap m_tmap_e{}, m_tmap_v{};
@@ -114,6 +127,9 @@ private:
     const float* m_map_e_ptr = nullptr;
     const float* m_map_v_ptr = nullptr;
     uint64_t m_map_batch = 1;
+    std::unique_ptr<RunFold> m_runs;  // run form, when the runs allow it
+    bool m_use_runs = false;
+    bool m_bound_groups = false;     // run form: the bound batch's segments are in groups
 };
 
 // One merge level: out[s, c] = rot(in[2s, tail(c)], st(c)) + rot(in[2s+1, head(c)], sh(c)).
