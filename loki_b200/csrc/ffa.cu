@@ -119,7 +119,7 @@ FFAExec::FFAExec(const Plan& p, int device, int storage, uint64_t max_batch_)
     sp = make_score_params(plan.widths.data(), static_cast<uint32_t>(plan.widths.size()),
                            static_cast<uint32_t>(plan.cfg.nbins));
     if (plan.nsegments[plan.n_levels - 1] == 1 &&
-        make_mask_score_params(sp, static_cast<uint32_t>(plan.cfg.nbins), &mp)) {
+        make_mask_score_params(sp, static_cast<uint32_t>(plan.cfg.nbins), &mp, true)) {
         wm = true;
         normtab.alloc(sizeof(float) * kNormTableSize);
         norm_table_fill(normtab.as<float>(), nullptr);

@@ -63,7 +63,7 @@ struct FFAExec {
     // BF16 search: per-cell best approximate S/N, the cells to rescore.
     DeviceBuffer cmax, cells, cell_vals, cell_count, cell_scratch;
     ScoreParams sp{};
-    // Final level for 32 / 64 / 128 bins and strictly increasing widths <= 32
+    // Final level for at most 128 bins and strictly increasing widths <= 32
     // (final_level.cu): width mask, 1 / sqrt(n) table, per-block candidate
     // counts and their offsets (FP32 search).
     bool wm = false;

@@ -150,7 +150,7 @@ struct ScoreParams {
 };
 ScoreParams make_score_params(const uint32_t* widths, uint32_t nwidths, uint32_t nbins);
 
-// ---- final level for 32 / 64 / 128 bins (final_level.cu) -----------------
+// ---- final level for at most 128 bins (final_level.cu) -------------------
 // 1 / sqrt(n) table for exact integer variance sums n < kNormTableSize
 // (rcp_rn(sqrt_rn(n)), the direct computation's bits).
 constexpr uint32_t kNormTableSize = 1u << 19;
@@ -165,9 +165,11 @@ struct MaskScoreParams {
     float b[33];
     uint8_t slot[33];
 };
-// False when the masked path does not apply (nbins not 32 / 64 / 128, widths
-// not strictly increasing or wider than 32 bins).
-bool make_mask_score_params(const ScoreParams& sp, uint32_t nbins, MaskScoreParams* mp);
+// False when the masked path does not apply (nbins not 32 / 64 / 128 -- or, for
+// the final level, any_nbins, above 128 -- widths not strictly increasing or
+// wider than 32 bins).
+bool make_mask_score_params(const ScoreParams& sp, uint32_t nbins, MaskScoreParams* mp,
+                            bool any_nbins = false);
 uint32_t final_level_cells_per_block();
 // Blocks (count slots) of one final-level launch.
 uint64_t final_level_blocks(uint64_t n_inner, uint64_t n_outer, uint64_t nbatch);

@@ -65,8 +65,8 @@ __global__ void score_kernel(const float* __restrict__ folds, uint64_t nprof, ui
 //
 // Phase 1 keeps many loads in flight: a warp takes PB profiles at a time,
 // loads their coordinates with one lane each, then issues every tail/head
-// load of the PB profiles (NJ = ceil(nbins / 32) bins per lane; NJ == 0
-// selects a generic loop for large nbins) before the first add.
+// load of the PB profiles (NJ = ceil(nbins / 32) bins per lane) before the
+// first add.
 template <bool TAYLOR, int NW, int NJ, int PB, class TIn, int NB>
 __global__ void merge_score_kernel(const TIn* __restrict__ in, const void* __restrict__ coords,
                                    uint32_t n_inner, uint32_t n_outer, uint64_t nprev,
@@ -89,24 +89,7 @@ __global__ void merge_score_kernel(const TIn* __restrict__ in, const void* __res
     const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     const uint32_t plen = 2 * nbins;
     const TIn* head_base = in + nprev * plen;  // segment 1 of the previous level
-    if constexpr (NJ == 0) {
-#pragma unroll 2
-        for (uint32_t p = warp; p < nhere; p += T / kWarp) {
-            const MergeCoord mc = load_merge_coord<TAYLOR>(coords, c0 + p, nbins);
-            const TIn* tail = in + static_cast<uint64_t>(mc.it) * plen;
-            const TIn* head = head_base + static_cast<uint64_t>(mc.ih) * plen;
-            float* dst = rows + static_cast<size_t>(p) * rs;
-            for (uint32_t j = lane; j < nbins; j += kWarp) {
-                const uint32_t jt = j >= mc.st ? j - mc.st : j + nbins - mc.st;
-                const uint32_t jh = j >= mc.sh ? j - mc.sh : j + nbins - mc.sh;
-                const float e = __fadd_rn(dev::Store<TIn>::load(tail + jt),
-                                          dev::Store<TIn>::load(head + jh));
-                const float v = __fadd_rn(dev::Store<TIn>::load(tail + nbins + jt),
-                                          dev::Store<TIn>::load(head + nbins + jh));
-                dst[j] = normalise(e, v);
-            }
-        }
-    } else {
+    {
         for (uint32_t p0 = warp * PB; p0 < nhere; p0 += (T / kWarp) * PB) {
             MergeCoord mine{0, 0, 0, 0};
             if (lane < PB && p0 + lane < nhere) {
@@ -175,6 +158,151 @@ __global__ void merge_score_kernel(const TIn* __restrict__ in, const void* __res
     }
 }
 
+// Wide profiles (nbins > 128): the rows of few cells fill shared memory, so a
+// thread per cell leaves an SM one or two warps (1024 bins: 32 cells a block,
+// one block an SM). Here a block of 8 warps shares R cells: only the prefix
+// sum, whose order of adds is fixed, is one thread per cell; the circular
+// extension and the window maxima go over all threads, a warp per cell with
+// its lanes over the positions. Maxima do not depend on the order except for
+// the sign of a zero, which is then taken from the reference's scan. Measured
+// on B200, 256 level-0 segments: 1024 bins (20 widths) 0.11 ms against 2.39,
+// 512 bins 0.20 against 1.95, 256 bins 0.61 against 1.50.
+constexpr uint32_t kWideThreads = 256;
+
+template <bool TAYLOR, int NW, class TIn>
+__global__ void __launch_bounds__(kWideThreads)
+    merge_score_wide_kernel(const TIn* __restrict__ in, const void* __restrict__ coords, uint32_t n_inner,
+                            uint32_t n_outer, uint64_t nprev, uint32_t nbins, uint32_t rs, uint32_t R, ScoreParams sp,
+                            int mode, float* __restrict__ scores, float* __restrict__ cmax) {
+    extern __shared__ float rows[];
+    in += static_cast<uint64_t>(blockIdx.y) * 2 * nprev * 2 * nbins;
+    scores += static_cast<uint64_t>(blockIdx.y) * n_inner * n_outer * (mode == LK_SCORE_PER_WIDTH ? sp.nwidths : 1);
+    if (cmax != nullptr) {
+        cmax += static_cast<uint64_t>(blockIdx.y) * n_inner * n_outer;
+    }
+    const uint32_t tile = blockIdx.x / n_outer;
+    const uint32_t outer = blockIdx.x - tile * n_outer;
+    const uint32_t j0 = tile * R;
+    const uint32_t nhere = min(R, n_inner - j0);
+    const uint64_t c0 = static_cast<uint64_t>(outer) * n_inner + j0;
+    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t plen = 2 * nbins;
+    const TIn* head_base = in + nprev * plen;
+    constexpr uint32_t U = 4;  // bins per lane with their loads in flight
+    for (uint32_t p = warp; p < nhere; p += kWideThreads / kWarp) {
+        const MergeCoord mc = load_merge_coord<TAYLOR>(coords, c0 + p, nbins);
+        const TIn* tail = in + static_cast<uint64_t>(mc.it) * plen;
+        const TIn* head = head_base + static_cast<uint64_t>(mc.ih) * plen;
+        float* dst = rows + static_cast<size_t>(p) * rs;
+        for (uint32_t b = lane; b < nbins; b += U * kWarp) {
+            float te[U], tv[U], he[U], hv[U];
+#pragma unroll
+            for (uint32_t k = 0; k < U; ++k) {
+                const uint32_t j = b + k * kWarp < nbins ? b + k * kWarp : b;
+                const uint32_t jt = j >= mc.st ? j - mc.st : j + nbins - mc.st;
+                const uint32_t jh = j >= mc.sh ? j - mc.sh : j + nbins - mc.sh;
+                te[k] = dev::Store<TIn>::load(tail + jt);
+                tv[k] = dev::Store<TIn>::load(tail + nbins + jt);
+                he[k] = dev::Store<TIn>::load(head + jh);
+                hv[k] = dev::Store<TIn>::load(head + nbins + jh);
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < U; ++k) {
+                if (b + k * kWarp < nbins) {
+                    dst[b + k * kWarp] = normalise(__fadd_rn(te[k], he[k]), __fadd_rn(tv[k], hv[k]));
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < nhere) {
+        float* r = rows + static_cast<size_t>(threadIdx.x) * rs;
+        float acc = r[0];
+        uint32_t j = 1;
+        for (; j + 8 <= nbins; j += 8) {
+            float x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                x[k] = r[j + k];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                acc = __fadd_rn(acc, x[k]);
+                r[j + k] = acc;
+            }
+        }
+        for (; j < nbins; ++j) {
+            acc = __fadd_rn(acc, r[j]);
+            r[j] = acc;
+        }
+    }
+    __syncthreads();
+    for (uint32_t p = warp; p < nhere; p += kWideThreads / kWarp) {
+        float* r = rows + static_cast<size_t>(p) * rs;
+        const float sum = r[nbins - 1];
+        for (uint32_t k = lane; k < sp.wmax; k += kWarp) {
+            r[nbins + k] = __fadd_rn(r[k], sum);
+        }
+        __syncwarp();
+        float dm[NW];
+#pragma unroll
+        for (int iw = 0; iw < NW; ++iw) {
+            dm[iw] = -FLT_MAX;
+        }
+        for (uint32_t i = lane; i < nbins; i += kWarp) {
+            const float ri = r[i];
+#pragma unroll
+            for (int iw = 0; iw < NW; ++iw) {
+                if (iw < static_cast<int>(sp.nwidths)) {
+                    dm[iw] = fmaxf(dm[iw], __fsub_rn(r[i + sp.widths[iw]], ri));
+                }
+            }
+        }
+        // lane iw takes width iw
+        float d = 0.0f, hb = 0.0f, b = 0.0f;
+        uint32_t w = 1;
+#pragma unroll
+        for (int iw = 0; iw < NW; ++iw) {
+            if (iw < static_cast<int>(sp.nwidths)) {
+                float m = dm[iw];
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+                }
+                if (static_cast<int>(lane) == iw) {
+                    d = m;
+                    hb = sp.hb[iw];
+                    b = sp.b[iw];
+                    w = sp.widths[iw];
+                }
+            }
+        }
+        if (lane < sp.nwidths && d == 0.0f) {
+            d = dmax_first(r, w, nbins);
+        }
+        const float snr = __fmul_rn(__fsub_rn(__fmul_rn(hb, d), __fmul_rn(b, sum)), 1.0f);
+        const uint64_t c = c0 + p;
+        if (mode == LK_SCORE_PER_WIDTH && lane < sp.nwidths) {
+            scores[c * sp.nwidths + lane] = snr;
+        }
+        if (mode == LK_SCORE_MAX || cmax != nullptr) {
+            float best = -FLT_MAX;
+            for (uint32_t iw = 0; iw < sp.nwidths; ++iw) {
+                const float v = __shfl_sync(0xffffffffu, snr, static_cast<int>(iw));
+                best = (best < v) ? v : best;
+            }
+            if (lane == 0) {
+                if (mode == LK_SCORE_MAX) {
+                    scores[c] = best;
+                }
+                if (cmax != nullptr) {
+                    cmax[c] = best;
+                }
+            }
+        }
+    }
+}
+
 }  // namespace
 
 // First parameter type of a merge_score_kernel instantiation.
@@ -239,6 +367,40 @@ void merge_score_level(const void* d_in, const void* d_coords, bool taylor, uint
     const uint32_t T = (cells_per_block >= 32 && cells_per_block % 32 == 0 && cells_per_block <= Tmax)
                            ? cells_per_block
                            : Tmax;
+    if (nbins > 128) {
+        // cells per block: rows in about 56 KB, four blocks an SM
+        uint32_t R = 32;
+        while (R > 8 && R * rs * sizeof(float) > 56 * 1024) {
+            R /= 2;
+        }
+        const size_t wsmem = static_cast<size_t>(R) * rs * sizeof(float);
+        const uint64_t wtiles = (n_inner + R - 1) / R;
+        require(wtiles * n_outer <= 0x7fffffffULL && n_inner <= 0xffffffffULL,
+                "final level too large for the launch grid");
+        auto wide = [&](auto tg, auto nwc, auto tin) {
+            using TIn = decltype(tin);
+            auto kern = merge_score_wide_kernel<decltype(tg)::value, decltype(nwc)::value, TIn>;
+            set_smem(kern, wsmem);
+            kern<<<dim3(static_cast<unsigned>(wtiles * n_outer), static_cast<unsigned>(nbatch)), kWideThreads, wsmem, s>>>(
+                static_cast<const TIn*>(d_in), d_coords, static_cast<uint32_t>(n_inner), static_cast<uint32_t>(n_outer),
+                ncoords_prev, nbins, rs, R, sp, mode, d_scores, d_cmax);
+        };
+        auto by_in = [&](auto tg, auto nwc) {
+            in_bf16 ? wide(tg, nwc, __nv_bfloat16{}) : wide(tg, nwc, float{});
+        };
+        auto by_nw = [&](auto tg) {
+            if (sp.nwidths <= 8) {
+                by_in(tg, std::integral_constant<int, 8>{});
+            } else if (sp.nwidths <= 16) {
+                by_in(tg, std::integral_constant<int, 16>{});
+            } else {
+                by_in(tg, std::integral_constant<int, 32>{});
+            }
+        };
+        taylor ? by_nw(std::true_type{}) : by_nw(std::false_type{});
+        LK_CUDA(cudaGetLastError());
+        return;
+    }
     const size_t smem = static_cast<size_t>(T) * rs * sizeof(float);
     const uint64_t tiles = (n_inner + T - 1) / T;
     require(tiles * n_outer <= 0x7fffffffULL && n_inner <= 0xffffffffULL,
@@ -254,7 +416,7 @@ void merge_score_level(const void* d_in, const void* d_coords, bool taylor, uint
             d_scores, d_cmax);
     };
     const int nwb = sp.nwidths <= 8 ? 8 : (sp.nwidths <= 16 ? 16 : 32);
-    const int nj = nbins <= 32 ? 1 : (nbins <= 64 ? 2 : (nbins <= 128 ? 4 : (nbins <= 256 ? 8 : 0)));
+    const int nj = nbins <= 32 ? 1 : (nbins <= 64 ? 2 : 4);
     // Dispatch (taylor, width bucket, bins per lane); PB * NJ = 16 loads of
     // each kind in flight per lane.
     auto pick = [&](auto tg, auto tin) {
@@ -272,13 +434,9 @@ void merge_score_level(const void* d_in, const void* d_coords, bool taylor, uint
             } else if (nj == 2) {
                 fixed ? launch(merge_score_kernel<TG, NWC, 2, 8, TI, 64 * FX>)
                       : launch(merge_score_kernel<TG, NWC, 2, 8, TI, 0>);
-            } else if (nj == 4) {
+            } else {
                 fixed ? launch(merge_score_kernel<TG, NWC, 4, 4, TI, 128 * FX>)
                       : launch(merge_score_kernel<TG, NWC, 4, 4, TI, 0>);
-            } else if (nj == 8) {
-                launch(merge_score_kernel<TG, NWC, 8, 2, TI, 0>);
-            } else {
-                launch(merge_score_kernel<TG, NWC, 0, 1, TI, 0>);
             }
         };
         if (nwb == 8) by_nj(std::integral_constant<int, 8>{});
