@@ -178,18 +178,32 @@ const void* FFAExec::run_levels(const float* ts_e, const float* ts_v, uint32_t l
     prof.begin(LK_STAGE_BRUTE_FOLD, 0, 1, series_bytes + 4 * plan.fold_size(0) * nbatch, s);
     bf->fold(static_cast<float*>(in), s, batch_lens);
     prof.end(s);
-    for (uint32_t l = 1; l <= last; ++l) {
-        void* out = (l == last && final_out != nullptr) ? final_out : buf[l % 2].ptr;
-        prof.begin(LK_STAGE_MERGE, static_cast<int>(l), 1,
-                   nbatch * (elem(l - 1) * plan.fold_size(l - 1) + elem(l) * plan.fold_size(l)) +
-                       coord_bytes(l),
+    // Levels in pairs, the first alone when their number is odd; levels
+    // alternate between the two buffers (a BF16 executor's first output, read
+    // from fold0, takes buf[1]).
+    int cur = 0;
+    for (uint32_t l = 1; l <= last;) {
+        const bool two = (last - l) % 2 == 1;
+        const uint32_t lo = two ? l + 1 : l;  // output level
+        void* out = (lo == last && final_out != nullptr) ? final_out : buf[1 - cur].ptr;
+        prof.begin(LK_STAGE_MERGE, static_cast<int>(lo), 1,
+                   nbatch * (elem(l - 1) * plan.fold_size(l - 1) + elem(lo) * plan.fold_size(lo)) +
+                       coord_bytes(lo) + (two ? coord_bytes(l) : 0),
                    s);
-        const uint64_t n_inner = plan.param_counts[l][plan.nparams - 1];
-        merge_level(in, out, level_coords(l), taylor, n_inner, plan.ncoords[l] / n_inner,
-                    plan.ncoords[l - 1], plan.nsegments[l] * nbatch, nbins, s, is_bf16(l - 1),
-                    is_bf16(l), merge_pb);
+        const uint64_t n_inner = plan.param_counts[lo][plan.nparams - 1];
+        if (two) {
+            merge_level2(in, out, level_coords(l), level_coords(lo), taylor, n_inner, plan.ncoords[lo] / n_inner,
+                         plan.ncoords[l - 1], plan.nsegments[lo] * nbatch, nbins, s, is_bf16(l - 1), is_bf16(l),
+                         is_bf16(lo));
+        } else {
+            merge_level(in, out, level_coords(l), taylor, n_inner, plan.ncoords[l] / n_inner,
+                        plan.ncoords[l - 1], plan.nsegments[l] * nbatch, nbins, s, is_bf16(l - 1),
+                        is_bf16(l), merge_pb);
+        }
         prof.end(s);
         in = out;
+        cur = 1 - cur;
+        l = lo + 1;
     }
     *last_bf16 = is_bf16(last);
     return in;

@@ -139,6 +139,13 @@ void merge_level(const void* d_in, void* d_out, const void* d_coords, bool taylo
                  uint64_t n_inner, uint64_t n_outer, uint64_t ncoords_prev, uint64_t nsegments,
                  uint32_t nbins, cudaStream_t s, bool in_bf16 = false, bool out_bf16 = false,
                  int pb = 0);
+// Two merge levels in one pass: coords_mid / coords are the tables of the level
+// between and of the output level (n_inner, n_outer, nsegments: the output
+// level's; ncoords_prev: the input level's cells). mid_bf16: the level between
+// is rounded to BF16 as if stored.
+void merge_level2(const void* d_in, void* d_out, const void* d_coords_mid, const void* d_coords, bool taylor,
+                  uint64_t n_inner, uint64_t n_outer, uint64_t ncoords_prev, uint64_t nsegments, uint32_t nbins,
+                  cudaStream_t s, bool in_bf16, bool mid_bf16, bool out_bf16);
 
 // Boxcar scoring parameters shared by the score kernels.
 struct ScoreParams {

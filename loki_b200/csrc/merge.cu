@@ -195,6 +195,97 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// Two levels in one pass: the rows of the level between are formed in
+// registers from their own two parents (the same adds in the same tree, rounded
+// to BF16 where that level is stored so) instead of being written and read
+// back. Levels of hundreds of MB are bound by that traffic (a level's reads of
+// shared parents hit L1 and L2): 2 x 8 merge levels of the 2^21-sample period
+// search at 128 bins take 1.33 ms against 1.86, those of the 2^22-sample
+// accelerated search 0.28 against 0.33; small levels save a launch each.
+// NB: nbins, or 0 at run time. PB rows per warp and UJ times 32 bins of each in
+// flight, eight loads an element.
+template <bool TAYLOR, class TIn, class TOut, bool MID16, int NB, int PB, int UJ>
+__global__ void __launch_bounds__(kThreads)
+    merge2_kernel(const TIn* __restrict__ in, TOut* __restrict__ out, const void* __restrict__ coords_mid,
+                  const void* __restrict__ coords, uint32_t n_inner, uint32_t n_outer, uint64_t nprev,
+                  uint32_t nbins_rt) {
+    const uint32_t nbins = NB > 0 ? static_cast<uint32_t>(NB) : nbins_rt;
+    const uint32_t row = 2 * nbins;
+    const uint32_t tile = blockIdx.x / n_outer;
+    const uint32_t outer = blockIdx.x - tile * n_outer;
+    const uint64_t s = blockIdx.y;
+    const uint64_t ncur = static_cast<uint64_t>(n_inner) * n_outer;
+    const uint32_t warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+    const uint32_t j0 = tile * kCoordsPerBlock;
+    const uint32_t j1 = min(j0 + kCoordsPerBlock, n_inner);
+    const uint64_t seg = nprev * row;
+    const TIn* base = in + 4 * s * seg;
+    TOut* out_base = out + (s * ncur + static_cast<uint64_t>(outer) * n_inner) * row;
+    // the sum of two rotations, each below nbins
+    auto turn = [&](uint32_t a, uint32_t b) -> uint32_t {
+        const uint32_t t = a + b;
+        return t >= nbins ? t - nbins : t;
+    };
+    for (uint32_t p0 = j0 + warp * PB; p0 < j1; p0 += (kThreads / kWarp) * PB) {
+        // lane 2 q: row q's tail half, lane 2 q + 1: its head half
+        uint32_t r0 = 0, r1 = 0, s0 = 0, s1 = 0;
+        if (lane < 2 * PB && p0 + lane / 2 < j1) {
+            const MergeCoord o =
+                load_merge_coord<TAYLOR>(coords, static_cast<uint64_t>(outer) * n_inner + p0 + lane / 2, nbins);
+            const bool head = (lane & 1u) != 0;
+            const MergeCoord m = load_merge_coord<TAYLOR>(coords_mid, head ? o.ih : o.it, nbins);
+            const uint32_t st = head ? o.sh : o.st;
+            r0 = m.it;
+            r1 = m.ih;
+            s0 = turn(m.st, st);
+            s1 = turn(m.sh, st);
+        }
+#pragma unroll 1
+        for (uint32_t b0 = 0; b0 < nbins; b0 += 32 * UJ) {
+            float e[PB][UJ][4], v[PB][UJ][4];
+#pragma unroll
+            for (int q = 0; q < PB; ++q) {
+                // (rows past j1 read row 0, in range, and are not stored)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t r = __shfl_sync(0xffffffffu, (h & 1) ? r1 : r0, 2 * q + h / 2);
+                    const uint32_t sh = __shfl_sync(0xffffffffu, (h & 1) ? s1 : s0, 2 * q + h / 2);
+                    const TIn* src = base + h * seg + static_cast<uint64_t>(r) * row;
+#pragma unroll
+                    for (int u = 0; u < UJ; ++u) {
+                        uint32_t j = b0 + lane + 32u * u;
+                        if constexpr (NB > 0) {
+                            j = (j - sh) & (NB - 1);
+                        } else {
+                            j = j < nbins ? j : 0u;
+                            j = j >= sh ? j - sh : j + nbins - sh;
+                        }
+                        e[q][u][h] = dev::Store<TIn>::load(src + j);
+                        v[q][u][h] = dev::Store<TIn>::load(src + nbins + j);
+                    }
+                }
+            }
+            auto mid = [](float x) {
+                return MID16 ? __bfloat162float(__float2bfloat16_rn(x)) : x;
+            };
+#pragma unroll
+            for (int q = 0; q < PB; ++q) {
+                TOut* o = out_base + static_cast<uint64_t>(p0 + q) * row;
+#pragma unroll
+                for (int u = 0; u < UJ; ++u) {
+                    const uint32_t j = b0 + lane + 32u * u;
+                    if (p0 + q < j1 && (NB > 0 || j < nbins)) {
+                        o[j] = dev::Store<TOut>::from_float(__fadd_rn(
+                            mid(__fadd_rn(e[q][u][0], e[q][u][1])), mid(__fadd_rn(e[q][u][2], e[q][u][3]))));
+                        o[nbins + j] = dev::Store<TOut>::from_float(__fadd_rn(
+                            mid(__fadd_rn(v[q][u][0], v[q][u][1])), mid(__fadd_rn(v[q][u][2], v[q][u][3]))));
+                    }
+                }
+            }
+        }
+    }
+}
+
 }  // namespace
 
 void merge_level(const void* d_in, void* d_out, const void* d_coords, bool taylor,
@@ -276,6 +367,58 @@ void merge_level(const void* d_in, void* d_out, const void* d_coords, bool taylo
         } else {
             launch(__nv_bfloat16{}, float{});
         }
+        LK_CUDA(cudaGetLastError());
+    }
+}
+
+void merge_level2(const void* d_in, void* d_out, const void* d_coords_mid, const void* d_coords, bool taylor,
+                  uint64_t n_inner, uint64_t n_outer, uint64_t ncoords_prev, uint64_t nsegments, uint32_t nbins,
+                  cudaStream_t s, bool in_bf16, bool mid_bf16, bool out_bf16) {
+    require(n_inner > 0 && n_outer > 0, "empty merge level");
+    const uint64_t tiles = (n_inner + kCoordsPerBlock - 1) / kCoordsPerBlock;
+    require(tiles * n_outer <= 0x7fffffffULL && n_inner <= 0xffffffffULL && n_outer <= 0xffffffffULL,
+            "merge level too large for the launch grid");
+    const uint64_t row = 2ull * nbins;
+    for (uint64_t seg0 = 0; seg0 < nsegments; seg0 += 65535) {
+        const uint64_t ns = std::min<uint64_t>(65535, nsegments - seg0);
+        dim3 grid(static_cast<unsigned>(tiles * n_outer), static_cast<unsigned>(ns));
+        auto launch = [&](auto tg, auto tin, auto tout, auto mid) {
+            constexpr bool TG = decltype(tg)::value;
+            constexpr bool M16 = decltype(mid)::value;
+            using TIn = decltype(tin);
+            using TOut = decltype(tout);
+            auto go = [&](auto kern) {
+                kern<<<grid, kThreads, 0, s>>>(static_cast<const TIn*>(d_in) + seg0 * 4 * ncoords_prev * row,
+                                               static_cast<TOut*>(d_out) + seg0 * n_inner * n_outer * row,
+                                               d_coords_mid, d_coords, static_cast<uint32_t>(n_inner),
+                                               static_cast<uint32_t>(n_outer), ncoords_prev, nbins);
+            };
+            switch (nbins) {
+                case 32: go(merge2_kernel<TG, TIn, TOut, M16, 32, 4, 1>); break;
+                case 64: go(merge2_kernel<TG, TIn, TOut, M16, 64, 2, 2>); break;
+                case 128: go(merge2_kernel<TG, TIn, TOut, M16, 128, 1, 4>); break;
+                case 256: go(merge2_kernel<TG, TIn, TOut, M16, 256, 1, 4>); break;
+                case 512: go(merge2_kernel<TG, TIn, TOut, M16, 512, 1, 4>); break;
+                case 1024: go(merge2_kernel<TG, TIn, TOut, M16, 1024, 1, 4>); break;
+                default:
+                    nbins <= 32   ? go(merge2_kernel<TG, TIn, TOut, M16, 0, 4, 1>)
+                    : nbins <= 64 ? go(merge2_kernel<TG, TIn, TOut, M16, 0, 2, 2>)
+                                  : go(merge2_kernel<TG, TIn, TOut, M16, 0, 1, 4>);
+            }
+        };
+        auto by_type = [&](auto tg) {
+            if (!mid_bf16) {
+                require(!in_bf16 && !out_bf16, "internal: FP32 between BF16 levels");
+                launch(tg, float{}, float{}, std::false_type{});
+            } else if (!in_bf16) {
+                out_bf16 ? launch(tg, float{}, __nv_bfloat16{}, std::true_type{})
+                         : launch(tg, float{}, float{}, std::true_type{});
+            } else {
+                out_bf16 ? launch(tg, __nv_bfloat16{}, __nv_bfloat16{}, std::true_type{})
+                         : launch(tg, __nv_bfloat16{}, float{}, std::true_type{});
+            }
+        };
+        taylor ? by_type(std::true_type{}) : by_type(std::false_type{});
         LK_CUDA(cudaGetLastError());
     }
 }
