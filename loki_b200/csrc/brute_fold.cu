@@ -1360,7 +1360,7 @@ void BruteFoldDevice::bind_inputs(const float* d_ts_e, const float* d_ts_v, cuda
         require(nbatch * m_nseg <= 0x7fffffffULL, "BruteFold: too many segments");
         m_bound_groups = make_groups(d_lens, nbatch, s);
         const uint32_t* tab = m_bound_groups ? m_groups.as<uint32_t>() : nullptr;
-        m_runs->transpose(d_ts_e, d_ts_v, nbatch * m_nseg, tab ? tab + 1 + nbatch : nullptr, tab, s);
+        m_runs->transpose(d_ts_e, d_ts_v, nbatch * m_nseg, m_warps, tab ? tab + 1 + nbatch : nullptr, tab, s);
         m_map_batch = nbatch;
         m_map_e_ptr = d_ts_e;  // marks the inputs as bound
         return;

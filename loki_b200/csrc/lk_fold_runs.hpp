@@ -68,21 +68,24 @@ public:
     // follows from the shared memory the sums leave).
     static uint32_t marker_stages();
     // Transposes nrows segments into [group of 32][sample][32 lanes] (e, v)
-    // pairs. groups / ngroups: the segment-group table (nullptr: all rows in
-    // order).
-    void transpose(const float* d_e, const float* d_v, uint64_t nrows, const uint32_t* groups,
+    // pairs, or groups of 64 with unit variances into pairs of their E, for a
+    // fold() of `warps` warps. groups / ngroups: the segment-group table
+    // (nullptr: all rows in order).
+    void transpose(const float* d_e, const float* d_v, uint64_t nrows, uint32_t warps, const uint32_t* groups,
                    const uint32_t* ngroups, cudaStream_t s);
     void fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t* groups,
               const uint32_t* ngroups, uint32_t* d_status, cudaStream_t s) const;
-    uint64_t device_bytes() const { return m_items.bytes + m_rots.bytes + m_bits.bytes + m_evt.bytes; }
+    uint64_t device_bytes() const { return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes; }
 
 private:
+    bool pairs_e(uint64_t nrows, uint32_t warps) const;
     bool m_ok = false;
+    bool m_unit = false;  // the transposed rows were checked for unit variances
     uint32_t m_nfreq, m_nbins, m_seglen;
     uint32_t m_nranges = 1, m_range = 0;  // bin ranges per frequency, bins per range
     uint32_t m_pad = 0;                   // zero samples before each segment
     uint32_t m_nstages = 0;               // stages of one padded segment
-    DeviceBuffer m_items, m_rots, m_bits, m_evt;
+    DeviceBuffer m_items, m_rots, m_bits, m_counts, m_varied, m_evt;
     uint32_t m_wpr = 1;
     uint64_t m_evt_groups = 0;
 };
