@@ -424,14 +424,15 @@ __global__ void __launch_bounds__(256)
                         uint32_t nrows, uint32_t seglen, uint32_t pad, uint32_t qlen, bool vec4,
                         const uint32_t* groups, const uint32_t* ngroups, const uint32_t* varied) {
     __shared__ float2 tile[kTile][33];
-    const uint32_t grp = blockIdx.y;
+    const uint32_t tiles = (seglen + kTile - 1) / kTile;
+    const uint32_t grp = blockIdx.x / tiles;
     if (varied != nullptr && varied[grp / 2] == 0) {
         return;  // laid out by pair_e_kernel
     }
     if (ngroups != nullptr && grp * 4u >= *ngroups) {
         return;
     }
-    const uint32_t s0 = blockIdx.x * kTile;
+    const uint32_t s0 = (blockIdx.x - grp * tiles) * kTile;
     const uint32_t j = threadIdx.x / 8, c = threadIdx.x % 8;
     uint32_t row = grp * 32u + j;
     bool have = row < nrows;
@@ -480,11 +481,12 @@ __global__ void __launch_bounds__(256)
                   uint32_t seglen, uint32_t pad, uint32_t qlen, bool vec4, const uint32_t* groups,
                   const uint32_t* ngroups, uint32_t* varied) {
     __shared__ float tile[kTile][65];
-    const uint32_t g64 = blockIdx.y;
+    const uint32_t tiles = (seglen + kTile - 1) / kTile;
+    const uint32_t g64 = blockIdx.x / tiles;
     if (ngroups != nullptr && g64 * 8u >= *ngroups) {
         return;
     }
-    const uint32_t s0 = blockIdx.x * kTile;
+    const uint32_t s0 = (blockIdx.x - g64 * tiles) * kTile;
     const uint32_t c = threadIdx.x % 8;
     bool ones = true;
 #pragma unroll
@@ -820,7 +822,8 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
                         const uint32_t* ngroups, cudaStream_t s) {
     const uint64_t ngrp = (nrows + 31) / 32;
     const uint64_t qlen = static_cast<uint64_t>(m_nstages) * kStageLen;
-    require(ngrp <= 65535, "BruteFold: too many segments");
+    const uint64_t tiles = (m_seglen + kTile - 1) / kTile;
+    require(ngrp * tiles <= 0x7fffffffULL, "BruteFold: too many segments");
     if (m_evt_groups < ngrp) {
         m_evt.alloc(ngrp * qlen * kSampleBytes);
         // the zeros before and after each segment stay; the samples between
@@ -829,7 +832,6 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
         m_evt_groups = ngrp;
     }
     const bool vec4 = (reinterpret_cast<uintptr_t>(d_e) % 16 == 0) && (reinterpret_cast<uintptr_t>(d_v) % 16 == 0);
-    dim3 grid((m_seglen + kTile - 1) / kTile, static_cast<unsigned>(ngrp));
     m_unit = pairs_e(nrows, warps);
     const uint64_t g64 = (nrows + 63) / 64;
     if (m_unit) {
@@ -837,12 +839,12 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
             m_varied.alloc(g64 * sizeof(uint32_t));
         }
         LK_CUDA(cudaMemsetAsync(m_varied.ptr, 0, g64 * sizeof(uint32_t), s));
-        pair_e_kernel<<<dim3(grid.x, static_cast<unsigned>(g64)), 256, 0, s>>>(
+        pair_e_kernel<<<static_cast<unsigned>(g64 * tiles), 256, 0, s>>>(
             d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen, m_pad, static_cast<uint32_t>(qlen),
             vec4, groups, ngroups, m_varied.as<uint32_t>());
         LK_CUDA(cudaGetLastError());
     }
-    transpose_ev_kernel<<<grid, 256, 0, s>>>(d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen,
+    transpose_ev_kernel<<<static_cast<unsigned>(ngrp * tiles), 256, 0, s>>>(d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen,
                                              m_pad, static_cast<uint32_t>(qlen), vec4, groups, ngroups,
                                              m_unit ? m_varied.as<uint32_t>() : nullptr);
     LK_CUDA(cudaGetLastError());
