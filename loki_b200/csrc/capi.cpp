@@ -188,6 +188,21 @@ void lk_ffa_destroy(lk_ffa* ffa) {
     }
 }
 
+int lk_ffa_levels_fit(const lk_plan* plan, int storage, uint32_t last, int has_output, int* fits) {
+    return guarded([&] {
+        need(plan, "plan");
+        need(fits, "fits");
+        const lk::Plan& p = plan->plan;
+        lk::require(last < p.n_levels, "level out of range");
+        *fits = 1;
+        try {
+            lk::ffa_level_steps(p, storage == LK_BF16, last, has_output != 0);
+        } catch (const lk::Error&) {
+            *fits = 0;
+        }
+    });
+}
+
 int lk_ffa_workspace_bytes(const lk_ffa* ffa, uint64_t* bytes) {
     return guarded([&] {
         need(ffa, "ffa");

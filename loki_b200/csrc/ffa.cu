@@ -48,6 +48,33 @@ StageProfiler::~StageProfiler() {
     }
 }
 
+uint64_t ffa_buffer_size(const Plan& plan, bool mixed) {
+    uint64_t n = 1;
+    for (uint32_t l = mixed ? 1 : 0; l + 1 < plan.n_levels; ++l) {
+        n = std::max(n, plan.fold_size(l));
+    }
+    return n;
+}
+
+// Levels in pairs, the first alone when their number is odd; levels alternate
+// between the two buffers (a BF16 executor's first output, read from fold0,
+// takes buf[1]).
+std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint32_t last, bool has_output) {
+    require(last < plan.n_levels, "internal: level out of range");
+    const uint64_t have = ffa_buffer_size(plan, mixed);
+    std::vector<LevelStep> steps;
+    int cur = 0;
+    for (uint32_t l = 1; l <= last;) {
+        const uint32_t to = (last - l) % 2 == 1 ? l + 1 : l;
+        const int dest = to == last && has_output ? -1 : 1 - cur;
+        require(dest < 0 || plan.fold_size(to) <= have, "a level of this plan needs the caller's output buffer");
+        steps.push_back({l - 1, to, dest});
+        cur = 1 - cur;
+        l = to + 1;
+    }
+    return steps;
+}
+
 FFAExec::FFAExec(const Plan& p, int device, int storage, uint64_t max_batch_)
     : plan(p), device(device), max_batch(max_batch_) {
     require(!plan.offsets_overflow, "coordinate offsets exceed 32 bits");
@@ -78,20 +105,14 @@ FFAExec::FFAExec(const Plan& p, int device, int storage, uint64_t max_batch_)
                                            plan.cfg.nbins, plan.cfg.nsamps, plan.cfg.tsamp,
                                            plan.t_ref0(), status.as<uint32_t>());
     if (!mixed) {
-        uint64_t inter = 0;  // largest level that is not the final one
-        for (uint32_t l = 0; l + 1 < plan.n_levels; ++l) {
-            inter = std::max(inter, plan.fold_size(l));
-        }
+        const uint64_t inter = ffa_buffer_size(plan, false);
         buf[0].alloc(sizeof(float) * inter * max_batch);
         buf[1].alloc(sizeof(float) * inter * max_batch);
     } else {
         const uint32_t L = plan.n_levels;
         require(L <= kRescoreMaxLevels && plan.nsegments[0] <= kRescoreMaxLeaves,
                 "BF16 storage supports at most 8192 level-0 segments");
-        uint64_t inter = 1;  // largest BF16 level (1 .. L-2)
-        for (uint32_t l = 1; l + 1 < L; ++l) {
-            inter = std::max(inter, plan.fold_size(l));
-        }
+        const uint64_t inter = ffa_buffer_size(plan, true);
         fold0.alloc(sizeof(float) * plan.fold_size(0) * max_batch);
         buf[0].alloc(2 * inter * max_batch);  // BF16
         buf[1].alloc(2 * inter * max_batch);
@@ -153,6 +174,7 @@ const void* FFAExec::run_levels(const float* ts_e, const float* ts_v, uint32_t l
                                float* final_out, cudaStream_t s, uint64_t nbatch,
                                bool* last_bf16) {
     require(nbatch >= 1 && nbatch <= max_batch, "nbatch must lie in [1, max_batch]");
+    const std::vector<LevelStep> steps = ffa_level_steps(plan, mixed, last, final_out != nullptr);
     const bool taylor = plan.nparams > 1;
     const auto nbins = static_cast<uint32_t>(plan.cfg.nbins);
     // Level l is BF16 when the storage is mixed, l >= 1, and it is not the
@@ -178,32 +200,26 @@ const void* FFAExec::run_levels(const float* ts_e, const float* ts_v, uint32_t l
     prof.begin(LK_STAGE_BRUTE_FOLD, 0, 1, series_bytes + 4 * plan.fold_size(0) * nbatch, s);
     bf->fold(static_cast<float*>(in), s, batch_lens);
     prof.end(s);
-    // Levels in pairs, the first alone when their number is odd; levels
-    // alternate between the two buffers (a BF16 executor's first output, read
-    // from fold0, takes buf[1]).
-    int cur = 0;
-    for (uint32_t l = 1; l <= last;) {
-        const bool two = (last - l) % 2 == 1;
-        const uint32_t lo = two ? l + 1 : l;  // output level
-        void* out = (lo == last && final_out != nullptr) ? final_out : buf[1 - cur].ptr;
+    for (const LevelStep& st : steps) {
+        const uint32_t lo = st.to;
+        const bool two = lo == st.from + 2;
+        void* out = st.dest < 0 ? final_out : buf[st.dest].ptr;
         prof.begin(LK_STAGE_MERGE, static_cast<int>(lo), 1,
-                   nbatch * (elem(l - 1) * plan.fold_size(l - 1) + elem(lo) * plan.fold_size(lo)) +
-                       coord_bytes(lo) + (two ? coord_bytes(l) : 0),
+                   nbatch * (elem(st.from) * plan.fold_size(st.from) + elem(lo) * plan.fold_size(lo)) +
+                       coord_bytes(lo) + (two ? coord_bytes(lo - 1) : 0),
                    s);
         const uint64_t n_inner = plan.param_counts[lo][plan.nparams - 1];
         if (two) {
-            merge_level2(in, out, level_coords(l), level_coords(lo), taylor, n_inner, plan.ncoords[lo] / n_inner,
-                         plan.ncoords[l - 1], plan.nsegments[lo] * nbatch, nbins, s, is_bf16(l - 1), is_bf16(l),
-                         is_bf16(lo));
+            merge_level2(in, out, level_coords(lo - 1), level_coords(lo), taylor, n_inner,
+                         plan.ncoords[lo] / n_inner, plan.ncoords[st.from], plan.nsegments[lo] * nbatch, nbins, s,
+                         is_bf16(st.from), is_bf16(lo - 1), is_bf16(lo));
         } else {
-            merge_level(in, out, level_coords(l), taylor, n_inner, plan.ncoords[l] / n_inner,
-                        plan.ncoords[l - 1], plan.nsegments[l] * nbatch, nbins, s, is_bf16(l - 1),
-                        is_bf16(l), merge_pb);
+            merge_level(in, out, level_coords(lo), taylor, n_inner, plan.ncoords[lo] / n_inner,
+                        plan.ncoords[st.from], plan.nsegments[lo] * nbatch, nbins, s, is_bf16(st.from),
+                        is_bf16(lo), merge_pb);
         }
         prof.end(s);
         in = out;
-        cur = 1 - cur;
-        l = lo + 1;
     }
     *last_bf16 = is_bf16(last);
     return in;
@@ -385,6 +401,7 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
     batch_lens = nullptr;
     lk_tuning best{};
     uint32_t tried = 0;
+    DeviceBuffer last_level;  // of a plan that stops at several segments
     // Median of reps timed passes (after one untimed pass) of the stages.
     auto time_stages = [&](std::initializer_list<int> kinds) {
         std::vector<float> t;
@@ -394,7 +411,7 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
                 scores_impl(ts_e, ts_v, scores_tmp.as<float>(), nullptr, s, 1);
             } else {
                 bool last_bf16 = false;
-                run_levels(ts_e, ts_v, plan.n_levels - 1, nullptr, s, 1, &last_bf16);
+                run_levels(ts_e, ts_v, plan.n_levels - 1, last_level.as<float>(), s, 1, &last_bf16);
             }
             LK_CUDA(cudaStreamSynchronize(s));
             if (r > 0) {
@@ -406,6 +423,9 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
         return t[t.size() / 2];
     };
     try {
+        if (!scoring) {
+            last_level.alloc(sizeof(float) * plan.fold_size(plan.n_levels - 1));
+        }
         // 1. brute fold (with the interleave pass when both rows share a warp)
         const uint32_t rows0 = bf->rows(), warps0 = bf->warps(), stages0 = bf->stages();
         float bf_best = INFINITY;

@@ -45,6 +45,20 @@ struct StageProfiler {
     ~StageProfiler();
 };
 
+// One launch of the level loop: the level it reads, the level it stores (one
+// or two further) and where: buf[dest], or the caller's output (dest < 0).
+struct LevelStep {
+    uint32_t from, to;
+    int dest;
+};
+// Elements (per series) of each of the two intermediate buffers: the largest
+// level before the last (with BF16 storage level 0 has its own).
+uint64_t ffa_buffer_size(const Plan& plan, bool mixed);
+// The merge launches of levels 1 .. last. Fails when a level does not fit the
+// buffer it would be stored in (the last level of a plan may be larger than
+// every level before it and then needs the caller's output).
+std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint32_t last, bool has_output);
+
 struct FFAExec {
     Plan plan;
     int device;

@@ -143,3 +143,24 @@ def test_params_dict_and_fold_shapes():
     assert plan.fold_size == int(np.prod(shp))
     strides = plan.param_cart_strides[-1]
     assert strides.tolist() == [plan.param_counts[-1][1], 1]
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("accel, bseg", [(20000.0, 2**17), (6000.0, 2**16)])
+def test_last_level_larger_than_the_buffers(bf16, accel, bseg):
+    """A plan that stops at several segments and whose last level is its
+    largest: only the caller's output holds that level."""
+    from loki_b200 import _capi as C
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.plans import FFAPlanTime
+
+    cfg = PulsarSearchConfig(2**18, 1e-3, 32, 1.0, np.array([[-accel, accel], [5.0, 6.0]]), use_fourier=False,
+                             bseg_ffa=bseg)
+    plan = FFAPlanTime(cfg)
+    sizes = [int(n) * int(c) * 64 for n, c in zip(plan.nsegments, plan.ncoords)]
+    assert plan.nsegments[-1] > 1 and sizes[-1] > 2 * max(sizes[:-1])
+    fits = ctypes.c_int(-1)
+    for last in range(plan.n_levels):
+        for has_output in (0, 1):
+            C.check(C.lib().lk_ffa_levels_fit(plan._handle, 1 if bf16 else 0, last, has_output, ctypes.byref(fits)))
+            assert fits.value == (1 if has_output or last + 1 < plan.n_levels else 0)

@@ -183,6 +183,28 @@ def test_autotune_multi_segment_plan(cuda):
     assert ffa.status() == 0
 
 
+@pytest.mark.parametrize("storage", ["fp32", "bf16"])
+@pytest.mark.parametrize("accel, bseg", [(20000.0, 2**17), (6000.0, 2**16)])
+def test_autotune_last_level_largest(cuda, accel, bseg, storage):
+    """Tuning a plan that stops at several segments and whose last level is
+    larger than the buffers of the levels before it (odd and even numbers of
+    merges): the timed passes store it in a buffer of its own."""
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.ffa import FFACUDA
+
+    ns, lims = 2**18, [[-accel, accel], [5.0, 6.0]]
+    cfg = PulsarSearchConfig(ns, 1e-3, 32, 1.0, np.array(lims), use_fourier=False, bseg_ffa=bseg)
+    e, v = series(ns, 94)
+    ffa = FFACUDA(cfg, fold_storage=storage)
+    want = ffa.execute(e, v)
+    ffa.autotune(e, v, reps=1)
+    np.testing.assert_array_equal(ffa.execute(e, v).view(np.uint32), want.view(np.uint32))
+    if storage == "fp32":
+        op = lko.plan_create(lko.make_cfg(ns, 1e-3, 32, 1.0, lims, bseg_ffa=bseg))
+        np.testing.assert_array_equal(want.view(np.uint32), lko.ffa(op, e, v).view(np.uint32))
+    assert ffa.status() == 0
+
+
 def test_multi_series_slots_identical(cuda):
     """Batches alternating over two executor slots (own streams, own graphs)
     give exactly the one-slot results; device inputs, several batches per
