@@ -1113,7 +1113,7 @@ std::vector<FoldRuns> fold_runs(const std::vector<double>& freqs, uint64_t segme
 
 BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segment_len,
                                  uint64_t nbins, uint64_t nsamps, double tsamp, double t_ref,
-                                 uint32_t* d_status)
+                                 uint32_t* d_status, uint64_t max_batch)
     : m_nfreq(freqs.size()),
       m_seglen(segment_len),
       m_nbins(nbins),
@@ -1121,6 +1121,7 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
       m_freqs(freqs),
       m_tsamp(tsamp),
       m_t_ref(t_ref),
+      m_max_batch(max_batch),
       m_status(d_status) {
     require(!freqs.empty(), "BruteFold: Frequency array is empty");
     require(segment_len > 0 && nsamps % segment_len == 0,
@@ -1163,22 +1164,38 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     }
     require(configure(rows, warps, stages),
             "BruteFold: nbins too large for the shared-memory accumulators");
-    m_runs = std::make_unique<RunFold>(fold_runs(freqs, segment_len, nbins, tsamp, t_ref), m_seglen, m_nbins);
+    m_runs = std::make_unique<RunFold>(fold_runs(freqs, segment_len, nbins, tsamp, t_ref), m_seglen, m_nbins,
+                                       m_max_batch * m_nseg);
     if (!m_runs->ok()) {
         m_runs.reset();
     } else if (std::getenv("LOKI_B200_BF_ROWS") == nullptr && std::getenv("LOKI_B200_BF_WARPS") == nullptr &&
                std::getenv("LOKI_B200_BF_STAGES") == nullptr) {
         configure(2, 0, run_form_stages());
     }
+    if (m_nseg % 8 == 0) {
+        m_groups.alloc((1 + m_max_batch + m_max_batch * m_nseg / 8) * sizeof(uint32_t));
+    }
     m_ready = true;
-    if (!m_use_runs) {
-        make_tables();
+    prepare(m_use_runs, m_rows);
+}
+
+void BruteFoldDevice::prepare(bool runs, uint32_t rows) {
+    if (!m_ready) {
+        return;
+    }
+    if (runs) {
+        m_runs->reserve();
+        return;
+    }
+    make_tables();
+    if (rows == 2 && m_ev.ptr == nullptr) {
+        m_ev.alloc(m_max_batch * m_nsamps * sizeof(float2));
     }
 }
 
 // Tables of the forms that walk samples (made when one of them is selected).
 void BruteFoldDevice::make_tables() {
-    if (!m_ready || m_masks.ptr != nullptr) {
+    if (m_masks.ptr != nullptr) {
         return;
     }
     // Run tables, one frequency per task (host threads; same arithmetic as
@@ -1258,6 +1275,7 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
         if (w == 0 || w > m_runs->max_warps() || m_runs->blocks_per_group(w) > 65535) {
             return false;
         }
+        prepare(true, rows);
         m_rows = rows;
         m_warps = w;
         m_stages = stages;
@@ -1284,6 +1302,7 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
         if (smem > kSmemLimit || (m_nfreq + warps - 1) / warps > 65535) {
             return false;
         }
+        prepare(false, rows);
         m_rows = rows;
         m_warps = warps;
         m_stages = stages;
@@ -1292,7 +1311,6 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
         // second block never waits for the first one's tensor memory
         m_smem = std::max<size_t>(smem, 116 * 1024);
         m_use_runs = false;
-        make_tables();
         m_map_e_ptr = nullptr;
         m_map_ev_ptr = nullptr;
         return true;
@@ -1322,13 +1340,13 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
     if (w < 1 || w > wmax || (nitems + w - 1) / w > 65535) {
         return false;
     }
+    prepare(false, rows);
     m_rows = rows;
     m_warps = w;
     m_stages = stages;
     m_tmem = 0;
     m_smem = ring + w * per_warp;
     m_use_runs = false;
-    make_tables();
     m_map_e_ptr = nullptr;  // the input binding depends on the rows
     m_map_ev_ptr = nullptr;
     return true;
@@ -1354,7 +1372,7 @@ uint64_t BruteFoldDevice::device_bytes() const {
 // nbatch * nseg segments: every segment is folded from its own start.
 void BruteFoldDevice::bind_inputs(const float* d_ts_e, const float* d_ts_v, cudaStream_t s,
                                   uint64_t nbatch, const uint64_t* d_lens) {
-    require(nbatch >= 1, "BruteFold: nbatch must be positive");
+    require(nbatch >= 1 && nbatch <= m_max_batch, "BruteFold: nbatch must lie in [1, max_batch]");
     const uint64_t n = nbatch * m_nsamps;
     if (m_use_runs) {
         require(nbatch * m_nseg <= 0x7fffffffULL, "BruteFold: too many segments");
@@ -1366,9 +1384,6 @@ void BruteFoldDevice::bind_inputs(const float* d_ts_e, const float* d_ts_v, cuda
         return;
     }
     if (m_rows == 2) {
-        if (m_ev.bytes < n * sizeof(float2)) {
-            m_ev.alloc(n * sizeof(float2));
-        }
         const bool vec4 = (reinterpret_cast<uintptr_t>(d_ts_e) % 16 == 0) &&
                           (reinterpret_cast<uintptr_t>(d_ts_v) % 16 == 0);
         int dev = 0, nsm = 148;
@@ -1393,8 +1408,8 @@ void BruteFoldDevice::bind_inputs(const float* d_ts_e, const float* d_ts_v, cuda
     const bool aligned = (reinterpret_cast<uintptr_t>(e) % 16 == 0) &&
                          (reinterpret_cast<uintptr_t>(v) % 16 == 0);
     if (!aligned) {
-        if (m_stage.bytes < 2 * n * sizeof(float)) {
-            m_stage.alloc(2 * n * sizeof(float));
+        if (m_stage.ptr == nullptr) {
+            m_stage.alloc(2 * m_max_batch * m_nsamps * sizeof(float));
         }
         float* se = m_stage.as<float>();
         float* sv = se + n;
@@ -1488,10 +1503,6 @@ void BruteFoldDevice::fold(float* d_fold, cudaStream_t s, const uint64_t* d_lens
 bool BruteFoldDevice::make_groups(const uint64_t* d_lens, uint64_t nbatch, cudaStream_t s) {
     if (d_lens == nullptr || m_rows != 2 || m_nseg % 8 != 0) {
         return false;
-    }
-    const uint64_t words = 1 + nbatch + nbatch * m_nseg / 8;
-    if (m_groups.bytes < words * sizeof(uint32_t)) {
-        m_groups.alloc(words * sizeof(uint32_t));
     }
     seg_groups_kernel<<<1, 256, 0, s>>>(d_lens, static_cast<uint32_t>(nbatch), static_cast<uint32_t>(m_nseg),
                                         m_seglen, m_groups.as<uint32_t>());

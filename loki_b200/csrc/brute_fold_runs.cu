@@ -706,10 +706,11 @@ RunTables build_tables(const std::vector<FoldRuns>& runs, uint64_t segment_len, 
 
 }  // namespace
 
-RunFold::RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins)
+RunFold::RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, uint64_t max_rows)
     : m_nfreq(static_cast<uint32_t>(runs.size())),
       m_nbins(static_cast<uint32_t>(nbins)),
-      m_seglen(static_cast<uint32_t>(segment_len)) {
+      m_seglen(static_cast<uint32_t>(segment_len)),
+      m_max_rows(max_rows) {
     const RunTables tb = build_tables(runs, segment_len, m_nbins);
     if (!tb.ok) {
         return;
@@ -818,26 +819,28 @@ bool RunFold::pairs_e(uint64_t nrows, uint32_t warps) const {
            (nrows + 31) / 32 * blocks_per_group(warps) > static_cast<uint64_t>(nsm);
 }
 
+void RunFold::reserve() {
+    if (m_evt.ptr != nullptr) {
+        return;
+    }
+    m_varied.alloc((m_max_rows + 63) / 64 * sizeof(uint32_t));
+    m_evt.alloc((m_max_rows + 31) / 32 * m_nstages * kStageBytes);
+    // the zeros before and after each segment stay; the samples between them
+    // are written by every call, on any stream
+    LK_CUDA(cudaMemsetAsync(m_evt.ptr, 0, m_evt.bytes, nullptr));
+    LK_CUDA(cudaStreamSynchronize(nullptr));
+}
+
 void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint32_t warps, const uint32_t* groups,
                         const uint32_t* ngroups, cudaStream_t s) {
     const uint64_t ngrp = (nrows + 31) / 32;
     const uint64_t qlen = static_cast<uint64_t>(m_nstages) * kStageLen;
     const uint64_t tiles = (m_seglen + kTile - 1) / kTile;
-    require(ngrp * tiles <= 0x7fffffffULL, "BruteFold: too many segments");
-    if (m_evt_groups < ngrp) {
-        m_evt.alloc(ngrp * qlen * kSampleBytes);
-        // the zeros before and after each segment stay; the samples between
-        // them are written by every call
-        LK_CUDA(cudaMemsetAsync(m_evt.ptr, 0, m_evt.bytes, s));
-        m_evt_groups = ngrp;
-    }
+    require(ngrp * tiles <= 0x7fffffffULL && nrows <= m_max_rows, "BruteFold: too many segments");
     const bool vec4 = (reinterpret_cast<uintptr_t>(d_e) % 16 == 0) && (reinterpret_cast<uintptr_t>(d_v) % 16 == 0);
     m_unit = pairs_e(nrows, warps);
     const uint64_t g64 = (nrows + 63) / 64;
     if (m_unit) {
-        if (m_varied.bytes < g64 * sizeof(uint32_t)) {
-            m_varied.alloc(g64 * sizeof(uint32_t));
-        }
         LK_CUDA(cudaMemsetAsync(m_varied.ptr, 0, g64 * sizeof(uint32_t), s));
         pair_e_kernel<<<static_cast<unsigned>(g64 * tiles), 256, 0, s>>>(
             d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen, m_pad, static_cast<uint32_t>(qlen),

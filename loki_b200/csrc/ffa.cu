@@ -103,7 +103,7 @@ FFAExec::FFAExec(const Plan& p, int device, int storage, uint64_t max_batch_)
     const uint32_t np = plan.nparams;
     bf = std::make_unique<BruteFoldDevice>(plan.param_grid(0, np - 1), plan.segment_lens[0],
                                            plan.cfg.nbins, plan.cfg.nsamps, plan.cfg.tsamp,
-                                           plan.t_ref0(), status.as<uint32_t>());
+                                           plan.t_ref0(), status.as<uint32_t>(), max_batch);
     if (!mixed) {
         const uint64_t inter = ffa_buffer_size(plan, false);
         buf[0].alloc(sizeof(float) * inter * max_batch);
@@ -273,6 +273,16 @@ void FFAExec::scores_impl(const float* ts_e, const float* ts_v, float* d_scores,
     prof.end(s);
 }
 
+// For max_batch series, on the first search: a buffer that a later call
+// replaced by a larger one would leave captured graphs on freed memory.
+void FFAExec::reserve_scores() {
+    if (compact_scratch.ptr == nullptr) {
+        const uint64_t most = plan.ncoords[plan.n_levels - 1] * plan.widths.size() * max_batch;
+        scores_tmp.alloc(most * sizeof(float));
+        compact_scratch.alloc(compact_scratch_bytes(most));
+    }
+}
+
 void FFAExec::search(const float* ts_e, const float* ts_v, float snr_min, uint32_t* d_idx,
                      float* d_snr, uint64_t max_cands, uint64_t* d_count, cudaStream_t s,
                      uint64_t nbatch) {
@@ -282,16 +292,14 @@ void FFAExec::search(const float* ts_e, const float* ts_v, float snr_min, uint32
     const uint64_t ncells = plan.ncoords[L - 1] * nbatch;
     const uint64_t n = ncells * plan.widths.size();
     DeviceGuard g(device);
-    if (scores_tmp.bytes < n * sizeof(float)) {
-        scores_tmp.alloc(n * sizeof(float));
-        compact_scratch.alloc(compact_scratch_bytes(n));
-    }
-    if (mixed && cmax.bytes < ncells * sizeof(float)) {
-        cmax.alloc(ncells * sizeof(float));
-        cells.alloc(ncells * sizeof(uint32_t));
-        cell_vals.alloc(ncells * sizeof(float));
+    reserve_scores();
+    if (mixed && cell_scratch.ptr == nullptr) {
+        const uint64_t most = plan.ncoords[L - 1] * max_batch;
+        cmax.alloc(most * sizeof(float));
+        cells.alloc(most * sizeof(uint32_t));
+        cell_vals.alloc(most * sizeof(float));
         cell_count.alloc(sizeof(uint64_t));
-        cell_scratch.alloc(compact_scratch_bytes(ncells));
+        cell_scratch.alloc(compact_scratch_bytes(most));
     }
     prof.reset();
     if (!mixed && use_wm()) {
@@ -300,9 +308,10 @@ void FFAExec::search(const float* ts_e, const float* ts_v, float snr_min, uint32
         const uint64_t n_inner = plan.param_counts[L - 1][plan.nparams - 1];
         const uint64_t n_outer = plan.ncoords[L - 1] / n_inner;
         const uint64_t nblk = final_level_blocks(n_inner, n_outer, nbatch);
-        if (blk_counts.bytes < nblk * sizeof(uint32_t)) {
-            blk_counts.alloc(nblk * sizeof(uint32_t));
-            blk_offsets.alloc(nblk * sizeof(uint64_t));
+        if (blk_offsets.ptr == nullptr) {
+            const uint64_t most = final_level_blocks(n_inner, n_outer, max_batch);
+            blk_counts.alloc(most * sizeof(uint32_t));
+            blk_offsets.alloc(most * sizeof(uint64_t));
         }
         scores_impl(ts_e, ts_v, scores_tmp.as<float>(), nullptr, s, nbatch, snr_min,
                     blk_counts.as<uint32_t>());
@@ -389,10 +398,8 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
     const bool scoring = plan.nsegments[plan.n_levels - 1] == 1;
     DeviceGuard g(device);
     reps = std::max<uint32_t>(1, std::min<uint32_t>(reps, 20));
-    const uint64_t n = plan.ncoords[plan.n_levels - 1] * plan.widths.size();
-    if (scoring && scores_tmp.bytes < n * sizeof(float)) {
-        scores_tmp.alloc(n * sizeof(float));
-        compact_scratch.alloc(compact_scratch_bytes(n));
+    if (scoring) {
+        reserve_scores();
     }
     const bool was_enabled = prof.enabled;
     prof.enabled = true;

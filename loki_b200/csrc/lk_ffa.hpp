@@ -138,6 +138,7 @@ struct FFAExec {
     void search(const float* ts_e, const float* ts_v, float snr_min, uint32_t* d_idx,
                 float* d_snr, uint64_t max_cands, uint64_t* d_count, cudaStream_t s,
                 uint64_t nbatch = 1);
+    void reserve_scores();
     uint32_t read_status(cudaStream_t s);
     // Cells the last BF16 search rescored (synchronises s).
     uint64_t rescored_cells(cudaStream_t s);

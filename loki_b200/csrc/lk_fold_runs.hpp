@@ -55,7 +55,8 @@ class RunFold {
 public:
     // Builds the tables; ok() is false when a frequency's runs do not have
     // the form the kernel takes (see brute_fold_runs.cu).
-    RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins);
+    // max_rows: most segments of a call.
+    RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, uint64_t max_rows);
     bool ok() const { return m_ok; }
     // Consumer warps per block the kernel allows, and the default for a fold
     // of nseg segments.
@@ -67,6 +68,9 @@ public:
     // Ring depth that names this form in a launch shape (its real depth
     // follows from the shared memory the sums leave).
     static uint32_t marker_stages();
+    // Allocates and clears the buffers of max_rows segments (on the first call
+    // only; they live as long as the object).
+    void reserve();
     // Transposes nrows segments into [group of 32][sample][32 lanes] (e, v)
     // pairs, or groups of 64 with unit variances into pairs of their E, for a
     // fold() of `warps` warps. groups / ngroups: the segment-group table
@@ -75,7 +79,9 @@ public:
                    const uint32_t* ngroups, cudaStream_t s);
     void fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t* groups,
               const uint32_t* ngroups, uint32_t* d_status, cudaStream_t s) const;
-    uint64_t device_bytes() const { return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes; }
+    uint64_t device_bytes() const {
+        return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes + m_varied.bytes;
+    }
 
 private:
     bool pairs_e(uint64_t nrows, uint32_t warps) const;
@@ -87,7 +93,7 @@ private:
     uint32_t m_nstages = 0;               // stages of one padded segment
     DeviceBuffer m_items, m_rots, m_bits, m_counts, m_varied, m_evt;
     uint32_t m_wpr = 1;
-    uint64_t m_evt_groups = 0;
+    uint64_t m_max_rows;
 };
 
 }  // namespace lk

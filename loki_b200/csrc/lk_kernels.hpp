@@ -50,7 +50,7 @@ class RunFold;
 class BruteFoldDevice {
 public:
     BruteFoldDevice(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
-                    uint64_t nsamps, double tsamp, double t_ref, uint32_t* d_status);
+                    uint64_t nsamps, double tsamp, double t_ref, uint32_t* d_status, uint64_t max_batch = 1);
     ~BruteFoldDevice();
     // Enqueue the fold of (d_ts_e, d_ts_v); d_fold must hold nseg * nfreq * 2 *
     // nbins floats.
@@ -58,8 +58,8 @@ public:
         bind_inputs(d_ts_e, d_ts_v, s);
         fold(d_fold, s);
     }
-    // Points the input tensor maps at the series, or at nbatch series of
-    // nsamps samples stored back to back. fold() then folds all of them:
+    // Points the input tensor maps at the series, or at nbatch (at most
+    // max_batch) series of nsamps samples stored back to back. fold() then folds all of them:
     // d_fold holds nbatch * fold_size() floats. With both rows per warp the
     // series are first interleaved into (e, v) pairs on `s` (one kernel; the
     // run form's transposition skips the segments past d_lens, see
@@ -100,9 +100,13 @@ private:
     // applies (see fold()); returns whether it does.
     bool make_groups(const uint64_t* d_lens, uint64_t nbatch, cudaStream_t s);
     void make_tables();
+    // Tables and buffers of a form, for max_batch series. Buffers are allocated
+    // here and freed with the object: a captured graph may hold their addresses.
+    void prepare(bool runs, uint32_t rows);
     uint64_t m_nfreq, m_seglen, m_nbins, m_nsamps, m_nseg = 0;
     std::vector<double> m_freqs;
     double m_tsamp, m_t_ref;
+    uint64_t m_max_batch;
     bool m_ready = false;      // the form has been chosen
     uint64_t m_nwords = 0;
     bool m_wide_bins = false;  // uint16 run bins (nbins > 256)

@@ -82,6 +82,58 @@ def test_batch_graph_replay(cuda):
     assert eager[0].numel() > 0
 
 
+@pytest.mark.parametrize("ones", [True, False])
+@pytest.mark.parametrize("nbins", [32, 64, 128, 256])
+def test_graph_of_a_smaller_batch_survives_a_larger_one(cuda, nbins, ones):
+    """A step of one series captured as the executor's first call, then eager
+    calls of four series (which must not replace buffers the graph holds),
+    then the graph again."""
+    from loki_b200.ffa import FFACUDA
+
+    t = cuda
+    n, nb = 1 << 17, 4
+    cfg = _cfg(n, nbins, ((20.0, 40.0),), tsamp=64e-6)
+    es, vs = (np.stack(x) for x in zip(*(series(n, 50 + k) for k in range(nb))))
+    e = t.from_numpy(es).cuda()
+    v = t.ones_like(e) if ones else t.from_numpy(vs).cuda()
+    want = FFACUDA(cfg, max_batch=nb).scores_batch(e, v).clone()  # loads the kernels too
+    flat = want.reshape(-1)
+    thr = float(np.quantile(flat.cpu().numpy(), 0.99))
+    ffa = FFACUDA(cfg, max_batch=nb)
+    size = ffa.workspace_bytes
+    out = t.empty_like(want[:1]).reshape(-1)
+    idx = t.empty(1 << 20, dtype=t.int32, device="cuda")
+    snr = t.empty(1 << 20, dtype=t.float32, device="cuda")
+    cnt = t.zeros(1, dtype=t.int64, device="cuda")
+    t.cuda.synchronize()
+    g = t.cuda.CUDAGraph()
+    with t.cuda.graph(g):
+        ffa.scores_batch(e[:1], v[:1], out)
+    assert ffa.workspace_bytes == size  # everything scores_batch needs is there from the start
+    ffa.search_batch(e[:1], v[:1], thr, idx, snr, cnt)
+    t.cuda.synchronize()
+    h = t.cuda.CUDAGraph()
+    with t.cuda.graph(h):
+        ffa.search_batch(e[:1], v[:1], thr, idx, snr, cnt)
+    size = ffa.workspace_bytes
+    assert t.equal(ffa.scores_batch(e, v), want)
+    total = ffa.search_batch(e, v, thr)[2]
+    assert total == int((flat >= thr).sum()) and ffa.workspace_bytes == size
+    for j in (2, 0, 3):
+        e[0].copy_(t.from_numpy(es[j]))
+        if not ones:
+            v[0].copy_(t.from_numpy(vs[j]))
+        g.replay()
+        h.replay()
+        t.cuda.synchronize()
+        assert t.equal(out, want[j])
+        keep = t.nonzero(want[j] >= thr).flatten()
+        assert int(cnt.item()) == keep.numel()
+        assert t.equal(idx[: keep.numel()], keep.to(t.int32)) and t.equal(snr[: keep.numel()], want[j][keep])
+    del g, h
+    assert ffa.status() == 0
+
+
 def test_multi_series_driver_matches_oracle(cuda):
     from loki_b200.batched import MultiSeriesSearch
 
