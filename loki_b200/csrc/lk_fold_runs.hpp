@@ -1,12 +1,10 @@
 // Run form of the brute fold (brute_fold_runs.cu): host tables and launch.
 #pragma once
 
-#include <algorithm>
-#include <atomic>
 #include <cstdint>
-#include <thread>
 #include <vector>
 
+#include "lk_host.hpp"
 #include "lk_kernels.hpp"
 
 namespace lk {
@@ -17,29 +15,6 @@ struct FoldRuns {
     std::vector<uint32_t> start;
     std::vector<uint16_t> bin;
 };
-
-// fn(i) for i < n on host threads: about one per 2^16 units of work (`each` per
-// item), at most 32.
-template <class F>
-void parallel_for(uint64_t n, uint64_t each, F&& fn) {
-    const uint64_t want = n * (each + 1) / 65536 + 1;
-    const auto nthreads = static_cast<unsigned>(
-        std::min<uint64_t>({want, n, 32, std::max(1u, std::thread::hardware_concurrency())}));
-    std::atomic<uint64_t> next{0};
-    auto work = [&] {
-        for (uint64_t i = next++; i < n; i = next++) {
-            fn(i);
-        }
-    };
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < nthreads; ++t) {
-        pool.emplace_back(work);
-    }
-    work();
-    for (auto& t : pool) {
-        t.join();
-    }
-}
 
 // Host replay of the run form's tables over one segment of one row (fold:
 // [nfreq][nbins]), with the kernel's reads checked against the padded segment;
