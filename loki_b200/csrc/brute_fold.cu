@@ -1070,45 +1070,61 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // operation of host_phase_bin is monotone in it. With at least two samples per
 // bin a run's end is therefore found from its expected place by stepping to the
 // sample where the bin changes, two evaluations a run instead of one a sample.
-std::vector<FoldRuns> fold_runs(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
-                                double tsamp, double t_ref) {
-    std::vector<FoldRuns> per_f(freqs.size());
-    parallel_for(freqs.size(), segment_len / 8, [&](uint64_t f) {
-        const double freq = freqs[f];
-        auto bin = [&](uint64_t i) {
-            return host_phase_bin((static_cast<double>(i) * tsamp) - t_ref, freq, nbins);
-        };
-        auto& rb = per_f[f];
-        const double step = freq * tsamp * static_cast<double>(nbins);  // bins per sample
-        const bool jump = step < 0.5;
-        double edge = 0.0;  // expected end of the current run, in samples
-        if (jump && step > 0.0) {
-            const double phase = -t_ref * freq;
-            const double at = (phase - std::floor(phase)) * static_cast<double>(nbins) + 0.5;
-            edge = (1.0 - (at - std::floor(at))) / step;
-            rb.start.reserve(static_cast<size_t>(static_cast<double>(segment_len) * step) + 8);
-            rb.bin.reserve(rb.start.capacity());
+// Runs and tables on 8 cores, walking every sample in brackets: 755 frequencies
+// of 16,384 samples, 64 bins 4.6 ms (19), 3,020 of 8,192, 128 bins 19 (49),
+// 1,200 of 1,024 at a bin a sample or more 2.8 (2.8).
+void fold_runs(double freq, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref, FoldRuns& rb) {
+    auto bin = [&](uint64_t i) { return host_phase_bin((static_cast<double>(i) * tsamp) - t_ref, freq, nbins); };
+    const double step = freq * tsamp * static_cast<double>(nbins);  // bins per sample
+    rb.start.clear();
+    rb.bin.clear();
+    if (!(step < 0.5)) {
+        // runs of a sample or two: every sample, without a branch on its bin
+        rb.start.resize(segment_len + 1);
+        rb.bin.resize(segment_len + 1);
+        uint32_t b = bin(0);
+        rb.start[0] = 0;
+        rb.bin[0] = static_cast<uint16_t>(b);
+        size_t n = 1;  // the entry past the runs so far is sample i's
+        for (uint64_t i = 1; i < segment_len; ++i) {
+            const uint32_t next = bin(i);
+            rb.start[n] = static_cast<uint32_t>(i);
+            rb.bin[n] = static_cast<uint16_t>(next);
+            n += next != b ? 1 : 0;
+            b = next;
         }
-        for (uint64_t i = 0; i < segment_len;) {
-            const uint32_t b = bin(i);
-            rb.start.push_back(static_cast<uint32_t>(i));
-            rb.bin.push_back(static_cast<uint16_t>(b));
-            uint64_t j = i + 1;
-            if (jump) {
-                const double g = step > 0.0 ? std::ceil(edge) : static_cast<double>(segment_len);
-                j = g > static_cast<double>(segment_len) ? segment_len : std::max(j, static_cast<uint64_t>(g));
-                while (j > i + 1 && bin(j - 1) != b) {
-                    --j;
-                }
-                edge += step > 0.0 ? 1.0 / step : 0.0;
+        rb.start.resize(n);
+        rb.bin.resize(n);
+        return;
+    }
+    rb.start.reserve(static_cast<size_t>(static_cast<double>(segment_len) * step) + 8);
+    rb.bin.reserve(rb.start.capacity());
+    const double phase = -t_ref * freq;
+    const double at = (phase - std::floor(phase)) * static_cast<double>(nbins) + 0.5;
+    const double last = static_cast<double>(segment_len);
+    // expected end of the current run, in samples (a frequency of 0 has one run)
+    double edge = step > 0.0 ? (1.0 - (at - std::floor(at))) / step : last;
+    uint32_t b = bin(0);  // of the run that starts at i
+    for (uint64_t i = 0; i < segment_len;) {
+        rb.start.push_back(static_cast<uint32_t>(i));
+        rb.bin.push_back(static_cast<uint16_t>(b));
+        uint64_t j = edge < last ? std::max(i + 1, static_cast<uint64_t>(std::ceil(edge))) : segment_len;
+        edge += 1.0 / step;
+        uint32_t after = b;  // bin of sample j, once it is known to differ
+        while (j > i + 1) {
+            const uint32_t before = bin(j - 1);
+            if (before == b) {
+                break;
             }
-            while (j < segment_len && bin(j) == b) {
-                ++j;
-            }
-            i = j;
+            after = before;
+            --j;
         }
-    });
-    return per_f;
+        while (after == b && j < segment_len && (after = bin(j)) == b) {
+            ++j;
+        }
+        i = j;
+        b = after;
+    }
 }
 
 BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segment_len,
@@ -1164,8 +1180,7 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     }
     require(configure(rows, warps, stages),
             "BruteFold: nbins too large for the shared-memory accumulators");
-    m_runs = std::make_unique<RunFold>(fold_runs(freqs, segment_len, nbins, tsamp, t_ref), m_seglen, m_nbins,
-                                       m_max_batch * m_nseg);
+    m_runs = std::make_unique<RunFold>(freqs, m_seglen, m_nbins, tsamp, t_ref, m_max_batch * m_nseg);
     if (!m_runs->ok()) {
         m_runs.reset();
     } else if (std::getenv("LOKI_B200_BF_ROWS") == nullptr && std::getenv("LOKI_B200_BF_WARPS") == nullptr &&
@@ -1200,7 +1215,10 @@ void BruteFoldDevice::make_tables() {
     }
     // Run tables, one frequency per task (host threads; same arithmetic as
     // the reference's BruteFold::compute_phase_time_domain, lib/fold.cpp:113-142).
-    const std::vector<FoldRuns> per_f = fold_runs(m_freqs, m_seglen, m_nbins, m_tsamp, m_t_ref);
+    std::vector<FoldRuns> per_f(m_nfreq);
+    parallel_for<int>(m_nfreq, fold_run_evaluations(m_freqs, m_tsamp, m_nbins, m_seglen), [&](uint64_t f, int&) {
+        fold_runs(m_freqs[f], m_seglen, m_nbins, m_tsamp, m_t_ref, per_f[f]);
+    });
     std::vector<uint32_t> masks(m_nfreq * m_nwords, 0u);
     for (uint64_t f = 0; f < m_nfreq; ++f) {
         for (const uint32_t i : per_f[f].start) {

@@ -55,6 +55,7 @@ constexpr uint32_t kMirror = 32;     // samples copied behind the ring: a unit's
 constexpr uint32_t kMinSlots = 4;
 constexpr uint32_t kMaxSlots = 12;
 constexpr uint32_t kRangeMax = 64;   // bins per warp
+static_assert(kRangeMax <= 64, "a rotation's longer runs are one 64-bit word");
 constexpr uint32_t kChunk = 16;      // run lengths below are compile-time: 2 runs (4 below 8) fit the mirror
 constexpr uint32_t kMaxLen = 2048;   // longest run
 constexpr uint32_t kMaxWarps = 20;
@@ -548,8 +549,9 @@ struct RunTables {
 };
 
 // The kernel's tables, or ok = false where it does not apply.
-RunTables build_tables(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint32_t nbins) {
-    const auto nfreq = static_cast<uint32_t>(runs.size());
+RunTables build_tables(const std::vector<double>& freqs, uint64_t segment_len, uint32_t nbins, double tsamp,
+                       double t_ref) {
+    const auto nfreq = static_cast<uint32_t>(freqs.size());
     const auto seglen = static_cast<uint32_t>(segment_len);
     RunTables tb;
     tb.nranges = (nbins + kRangeMax - 1) / kRangeMax;
@@ -559,51 +561,58 @@ RunTables build_tables(const std::vector<FoldRuns>& runs, uint64_t segment_len, 
     if (segment_len > (1u << 30) || segment_len % 4 != 0) {
         return tb;
     }
-    // Per frequency: the run length L, where the first run (made up to at
-    // least L samples, as the last one) starts, and whether bins step by one.
+    // Of one frequency: the run length L and, range after range, its rotations
+    // (first samples without the padding).
     struct Freq {
         bool ok = false;
-        bool seq = true;
         uint32_t len = 0;
-        int64_t first = 0;
-        std::vector<std::vector<uint32_t>> rots, bits;  // of each range
         std::vector<RunItem> items;
+        std::vector<int64_t> rots;
+        std::vector<uint32_t> bits;
+    };
+    // A thread's scratch: the runs, and the rotations of each range so far.
+    struct Scratch {
+        FoldRuns runs;
+        std::vector<uint32_t> cnt;
+        std::vector<std::vector<int64_t>> rots;
+        std::vector<std::vector<uint64_t>> longer;
     };
     std::vector<Freq> fr(nfreq);
-    const uint64_t each = runs.empty() ? 0 : runs[0].start.size() * 4;
-    parallel_for(nfreq, each, [&](uint64_t f) {
-        const auto& st = runs[f].start;
-        const auto& bn = runs[f].bin;
+    tb.counts.resize(static_cast<size_t>(nfreq) * nbins);
+    const uint32_t ng = tb.range / 4;
+    parallel_for<Scratch>(nfreq, fold_run_evaluations(freqs, tsamp, nbins, segment_len), [&](uint64_t f, Scratch& sc) {
+        fold_runs(freqs[f], segment_len, nbins, tsamp, t_ref, sc.runs);
+        const auto& st = sc.runs.start;
+        const auto& bn = sc.runs.bin;
         const size_t n = st.size();
-        Freq& x = fr[f];
-        if (n == 0) {
-            return;
-        }
         auto len_of = [&](size_t j) { return (j + 1 < n ? st[j + 1] : seglen) - st[j]; };
         uint32_t lo = 0xffffffffu, hi = 0;
-        for (size_t j = 0; j + 1 < n; ++j) {
-            x.seq = x.seq && bn[j + 1] == (bn[j] + 1u) % nbins;
-            if (j > 0) {
-                lo = std::min(lo, len_of(j));
-                hi = std::max(hi, len_of(j));
+        for (size_t j = 1; j + 1 < n; ++j) {
+            const uint32_t len = st[j + 1] - st[j];
+            lo = std::min(lo, len);
+            hi = std::max(hi, len);
+        }
+        bool seq = true;  // bins step by one
+        size_t rotations = 1, last_start = 0;
+        for (size_t j = 1; j < n; ++j) {
+            if (bn[j] <= bn[j - 1]) {
+                seq &= bn[j] == 0 && bn[j - 1] == nbins - 1;
+                last_start = j;
+                ++rotations;
+            } else {
+                seq &= bn[j] == bn[j - 1] + 1u;
             }
         }
         const uint32_t c0 = len_of(0), c1 = len_of(n - 1);
-        if (!x.seq) {
+        uint32_t len = 0;
+        int64_t first = 0;  // where the first run, made up to at least L samples, starts
+        if (!seq) {
             // Bins are skipped: every run is one sample and every other bin
             // none (L = 0). Frequencies near the sampling rate, whose
             // rotations hold a sample or two, are left to the other forms.
-            if ((n > 2 && hi > 1) || c0 > 1 || c1 > 1) {
+            if ((n > 2 && hi > 1) || c0 > 1 || c1 > 1 || rotations > seglen / 4 + 1) {
                 return;
             }
-            uint64_t rotations = 1;
-            for (size_t j = 1; j < n; ++j) {
-                rotations += bn[j] <= bn[j - 1];
-            }
-            if (rotations > seglen / 4 + 1) {
-                return;
-            }
-            x.len = 0;
         } else {
             if (n <= 2) {
                 lo = hi = std::max(c0, c1);
@@ -611,94 +620,91 @@ RunTables build_tables(const std::vector<FoldRuns>& runs, uint64_t segment_len, 
             if (hi > lo + 1 || c0 > lo + 1 || c1 > lo + 1 || lo + 1 > kMaxLen) {
                 return;
             }
-            x.len = lo;
-            x.first = n > 1 ? static_cast<int64_t>(st[1]) - std::max(c0, lo) : 0;
+            len = lo;
+            first = n > 1 ? static_cast<int64_t>(st[1]) - std::max(c0, lo) : 0;
+        }
+        sc.cnt.assign(nbins, 0);
+        sc.rots.resize(tb.nranges);
+        sc.longer.resize(tb.nranges);
+        Freq x;
+        x.len = len;
+        x.items.resize(tb.nranges);
+        for (uint32_t rg = 0; rg < tb.nranges; ++rg) {
+            sc.rots[rg].clear();
+            sc.longer[rg].clear();
+            x.items[rg] = RunItem{};
+            x.items[rg].len = len;
+            x.items[rg].bins = std::min(tb.range, nbins - rg * tb.range);
+        }
+        for (size_t k = 0; k < n;) {  // one rotation of one range
+            const uint32_t rg = bn[k] / tb.range;
+            const uint32_t rg0 = rg * tb.range, rg_end = rg0 + tb.range;
+            RunItem& it = x.items[rg];
+            int64_t pos = st[k];
+            if (seq && k == 0) {
+                // the first run, from the first bin of its group
+                pos = first - static_cast<int64_t>((bn[k] - rg0) % 4) * len;
+                it.t0 = (bn[k] - rg0) / 4;
+            }
+            uint64_t longer = 0;  // bit per bin: a run of more than L samples
+            uint32_t b = bn[k], next = b;
+            do {
+                b = next;
+                const uint32_t cur = (k + 1 < n ? st[k + 1] : seglen) - st[k];
+                sc.cnt[b] += cur;
+                longer |= static_cast<uint64_t>(cur > len) << (b - rg0);
+                next = ++k < n ? bn[k] : 0;
+            } while (next > b && next < rg_end);
+            it.t1 = seq && k > last_start ? (b - rg0) / 4 + 1 : ng;
+            sc.rots[rg].push_back(pos);
+            sc.longer[rg].push_back(longer);
+        }
+        std::copy(sc.cnt.begin(), sc.cnt.end(), tb.counts.begin() + f * nbins);
+        for (uint32_t rg = 0; rg < tb.nranges; ++rg) {
+            x.items[rg].nrot = static_cast<uint32_t>(sc.rots[rg].size());
+            x.rots.insert(x.rots.end(), sc.rots[rg].begin(), sc.rots[rg].end());
+            for (const uint64_t w : sc.longer[rg]) {
+                x.bits.push_back(static_cast<uint32_t>(w));
+                if (tb.wpr == 2) {
+                    x.bits.push_back(static_cast<uint32_t>(w >> 32));
+                }
+            }
         }
         x.ok = true;
+        fr[f] = std::move(x);
     });
     uint32_t lmax = 0;
+    size_t total = 0;
     for (const Freq& x : fr) {
         if (!x.ok) {
             return tb;
         }
         lmax = std::max(lmax, x.len + 1);
+        total += x.rots.size();
     }
     // A group of 4 bins reaches up to 4 runs before the segment's first
     // sample and past its last one.
     const uint32_t reach = 4 * lmax + kChunk;
     tb.pad = (reach + kStageLen - 1) / kStageLen * kStageLen;
     tb.nstages = (tb.pad + seglen + reach + kStageLen - 1) / kStageLen;
-
-    const uint32_t ng = tb.range / 4;
-    tb.counts.resize(static_cast<size_t>(nfreq) * nbins);
-    parallel_for(nfreq, each, [&](uint64_t f) {
-        const auto& st = runs[f].start;
-        const auto& bn = runs[f].bin;
-        const size_t n = st.size();
-        Freq& x = fr[f];
-        std::vector<uint32_t> cnt(nbins, 0);
-        for (size_t k = 0; k < n; ++k) {
-            cnt[bn[k]] += (k + 1 < n ? st[k + 1] : seglen) - st[k];
-        }
-        std::copy(cnt.begin(), cnt.end(), tb.counts.begin() + f * nbins);
-        x.rots.resize(tb.nranges);
-        x.bits.resize(tb.nranges);
-        x.items.resize(tb.nranges);
-        for (uint32_t rg = 0; rg < tb.nranges; ++rg) {
-            x.items[rg] = RunItem{};
-            x.items[rg].len = x.len;
-            x.items[rg].bins = std::min(tb.range, nbins - rg * tb.range);
-        }
-        uint32_t cur = 0;  // range of the rotation entry being filled
-        size_t last_start = n - 1;  // first run of the last rotation
-        while (last_start > 0 && bn[last_start] > bn[last_start - 1]) {
-            --last_start;
-        }
-        for (size_t k = 0; k < n; ++k) {
-            const uint32_t rg = bn[k] / tb.range, rel = bn[k] - rg * tb.range;
-            RunItem& it = x.items[rg];
-            if (k == 0 || rg != cur || bn[k] <= bn[k - 1]) {
-                int64_t pos = st[k];
-                if (x.seq && k == 0) {
-                    // the first run, from the first bin of its group
-                    pos = x.first - static_cast<int64_t>(rel % 4) * x.len;
-                    it.t0 = rel / 4;
-                }
-                x.rots[rg].push_back(static_cast<uint32_t>(pos + tb.pad));
-                x.bits[rg].resize(x.bits[rg].size() + tb.wpr, 0u);
-                ++it.nrot;
-                cur = rg;
-            }
-            if (std::max((k + 1 < n ? st[k + 1] : seglen) - st[k], x.len) > x.len) {
-                x.bits[rg][x.bits[rg].size() - tb.wpr + rel / 32] |= 1u << (rel % 32);
-            }
-            it.t1 = x.seq && k >= last_start ? rel / 4 + 1 : ng;
-        }
-    });
-    tb.items.resize(static_cast<size_t>(tb.nranges) * nfreq);
-    size_t total = 0;
-    for (uint32_t f = 0; f < nfreq; ++f) {
-        for (uint32_t rg = 0; rg < tb.nranges; ++rg) {
-            fr[f].items[rg].rot0 = static_cast<uint32_t>(total);
-            tb.items[static_cast<size_t>(rg) * nfreq + f] = fr[f].items[rg];
-            total += fr[f].rots[rg].size();
-        }
-    }
     if (total > 0x7fffffffULL) {
         return tb;
     }
-    tb.rots.resize(total);
-    tb.bits.resize(total * tb.wpr);
-    parallel_for(nfreq, each, [&](uint64_t f) {
+    tb.items.resize(static_cast<size_t>(tb.nranges) * nfreq);
+    tb.rots.reserve(std::max<size_t>(total, 1));
+    tb.bits.reserve(std::max<size_t>(total, 1) * tb.wpr);
+    for (uint32_t f = 0; f < nfreq; ++f) {
+        uint32_t at = static_cast<uint32_t>(tb.rots.size());
         for (uint32_t rg = 0; rg < tb.nranges; ++rg) {
-            const size_t at = fr[f].items[rg].rot0;
-            std::copy(fr[f].rots[rg].begin(), fr[f].rots[rg].end(), tb.rots.begin() + at);
-            std::copy(fr[f].bits[rg].begin(), fr[f].bits[rg].end(), tb.bits.begin() + at * tb.wpr);
+            RunItem& it = tb.items[static_cast<size_t>(rg) * nfreq + f];
+            it = fr[f].items[rg];
+            it.rot0 = at;
+            at += it.nrot;
         }
-    });
-    if (total == 0) {
-        tb.rots.push_back(0);
-        tb.bits.assign(tb.wpr, 0);
+        for (const int64_t pos : fr[f].rots) {
+            tb.rots.push_back(static_cast<uint32_t>(pos + tb.pad));
+        }
+        tb.bits.insert(tb.bits.end(), fr[f].bits.begin(), fr[f].bits.end());
     }
     tb.ok = true;
     return tb;
@@ -706,12 +712,13 @@ RunTables build_tables(const std::vector<FoldRuns>& runs, uint64_t segment_len, 
 
 }  // namespace
 
-RunFold::RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, uint64_t max_rows)
-    : m_nfreq(static_cast<uint32_t>(runs.size())),
+RunFold::RunFold(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref,
+                 uint64_t max_rows)
+    : m_nfreq(static_cast<uint32_t>(freqs.size())),
       m_nbins(static_cast<uint32_t>(nbins)),
       m_seglen(static_cast<uint32_t>(segment_len)),
       m_max_rows(max_rows) {
-    const RunTables tb = build_tables(runs, segment_len, m_nbins);
+    const RunTables tb = build_tables(freqs, segment_len, m_nbins, tsamp, t_ref);
     if (!tb.ok) {
         return;
     }
@@ -731,10 +738,10 @@ RunFold::RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64
     m_ok = true;
 }
 
-bool run_fold_replay(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, const float* ts,
-                     float* fold) {
-    const auto nfreq = static_cast<uint32_t>(runs.size());
-    const RunTables tb = build_tables(runs, segment_len, static_cast<uint32_t>(nbins));
+bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp,
+                     double t_ref, const float* ts, float* fold) {
+    const auto nfreq = static_cast<uint32_t>(freqs.size());
+    const RunTables tb = build_tables(freqs, segment_len, static_cast<uint32_t>(nbins), tsamp, t_ref);
     if (!tb.ok) {
         return false;
     }

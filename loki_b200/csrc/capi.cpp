@@ -772,8 +772,10 @@ int lk_brute_fold_replay(const double* freqs, uint64_t nfreqs, uint64_t segment_
         need(fold, "fold");
         need(applies, "applies");
         lk::require(segment_len > 0 && nbins >= 1 && nbins <= 65535, "BruteFold: bad segment length or nbins");
-        const auto runs = lk::fold_runs(std::vector<double>(freqs, freqs + nfreqs), segment_len, nbins, tsamp, t_ref);
-        *applies = lk::run_fold_replay(runs, segment_len, nbins, ts, fold) ? 1 : 0;
+        lk::require(nfreqs >= 1 && std::all_of(freqs, freqs + nfreqs, [](double f) { return f >= 0.0; }),
+                    "Frequency must be positive");
+        const std::vector<double> f(freqs, freqs + nfreqs);
+        *applies = lk::run_fold_replay(f, segment_len, nbins, tsamp, t_ref, ts, fold) ? 1 : 0;
     });
 }
 

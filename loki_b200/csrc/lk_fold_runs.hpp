@@ -16,22 +16,22 @@ struct FoldRuns {
     std::vector<uint16_t> bin;
 };
 
+// The runs of one frequency.
+void fold_runs(double freq, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref, FoldRuns& out);
+
 // Host replay of the run form's tables over one segment of one row (fold:
 // [nfreq][nbins]), with the kernel's reads checked against the padded segment;
 // false where the form does not apply.
-bool run_fold_replay(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, const float* ts,
-                     float* fold);
-
-// Run table of every frequency (host threads).
-std::vector<FoldRuns> fold_runs(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins,
-                                double tsamp, double t_ref);
+bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp,
+                     double t_ref, const float* ts, float* fold);
 
 class RunFold {
 public:
     // Builds the tables; ok() is false when a frequency's runs do not have
     // the form the kernel takes (see brute_fold_runs.cu).
     // max_rows: most segments of a call.
-    RunFold(const std::vector<FoldRuns>& runs, uint64_t segment_len, uint64_t nbins, uint64_t max_rows);
+    RunFold(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref,
+            uint64_t max_rows);
     bool ok() const { return m_ok; }
     // Consumer warps per block the kernel allows, and the default for a fold
     // of nseg segments.
