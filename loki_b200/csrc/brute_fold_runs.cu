@@ -783,6 +783,17 @@ bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uin
 
 uint32_t RunFold::marker_stages() { return 32; }
 
+namespace {
+
+uint32_t sm_count() {
+    int dev = 0, nsm = 148;
+    LK_CUDA(cudaGetDevice(&dev));
+    LK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    return static_cast<uint32_t>(nsm);
+}
+
+}  // namespace
+
 uint32_t RunFold::max_warps() const {
     const size_t fixed = smem_bytes(kMinSlots, 0, 0);
     return static_cast<uint32_t>(std::min<size_t>((kSmemLimit - fixed) / (m_range * kSampleBytes), kMaxWarps));
@@ -791,20 +802,24 @@ uint32_t RunFold::max_warps() const {
 // A wave of blocks takes time in proportion to about 4 + its warps (2^22-sample
 // accelerated workload, nbins 64: 0.181 ms a wave with 5 warps, 0.191 with 6,
 // 0.270 with 11; 64 segments of 50 frequencies, one wave: 0.023 ms with 5,
-// 0.029 with 10, 0.050 with 20), so the fewest waves x (4 + warps).
+// 0.029 with 10, 0.050 with 20). Series with unit variances take half the
+// blocks of others, and which it will be is not known here: the warps with the
+// smallest product of the two costs (waves x (4 + warps)). Over 25 plans (32 to
+// 256 bins, 2^16 to 2^22 samples) that is on average 1.1 % above the best warps
+// with unit variances and 3.0 % with others; the smallest cost with unit
+// variances alone measured 1.9 and 7.1 %.
 uint32_t RunFold::default_warps(uint64_t nseg) const {
-    int dev = 0, nsm = 148;
-    LK_CUDA(cudaGetDevice(&dev));
-    LK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const uint64_t xblocks = (nseg + 63) / 64;  // unit variances, the usual series
+    const uint32_t nsm = sm_count();
     uint64_t best = ~0ull;
     uint32_t w = 0;  // none: more blocks than a launch takes
     const uint32_t wmax = max_warps();
     for (uint32_t c = std::min(wmax, 4u); c <= wmax; ++c) {
-        const uint64_t blocks = xblocks * m_nranges * ((m_nfreq + c - 1) / c);
-        const uint64_t cost = (blocks + nsm - 1) / nsm * (4 + c);
-        if (blocks / xblocks <= 65535 && cost < best) {
-            best = cost;
+        const uint64_t per_group = blocks_per_group(c);
+        auto cost = [&](uint64_t groups) { return (groups * per_group + nsm - 1) / nsm * (4 + c); };
+        const uint64_t varied = cost((nseg + 31) / 32);
+        const uint64_t unit = pairs_e(nseg, c) ? cost((nseg + 63) / 64) : varied;
+        if (per_group <= 65535 && varied * unit < best) {
+            best = varied * unit;
             w = c;
         }
     }
@@ -819,11 +834,7 @@ uint32_t RunFold::default_warps(uint64_t nseg) const {
 // blocks would take the same time with half the groups, so the check and its
 // launches are left out there.
 bool RunFold::pairs_e(uint64_t nrows, uint32_t warps) const {
-    int dev = 0, nsm = 148;
-    LK_CUDA(cudaGetDevice(&dev));
-    LK_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    return nrows > 32 && m_seglen <= (1u << 24) &&
-           (nrows + 31) / 32 * blocks_per_group(warps) > static_cast<uint64_t>(nsm);
+    return nrows > 32 && m_seglen <= (1u << 24) && (nrows + 31) / 32 * blocks_per_group(warps) > sm_count();
 }
 
 void RunFold::reserve() {
