@@ -371,7 +371,10 @@ int lk_sweep_results(const lk_sweep* sw, double* params, float* scores, uint64_t
 /* Launch-shape tuning (an autotuner of this library; no reference counterpart).
  * bf_*: brute fold rows (E, V) per consumer warp (1 or 2), consumer warps
  * per block (0: the wave-count rule), shared-memory ring depth in 32-sample
- * words (32: the run form, whose depth follows from the memory its sums leave);
+ * words (32: the run form, whose depth follows from the memory its sums leave).
+ * Fields at 0 keep the present value or the rule; while the run form is in use
+ * or named, a shape that it does not take (one row, more warps, TMEM warps) goes
+ * to the form that walks samples;
  * merge_rows_in_flight: output rows per warp whose loads are issued
  * together in a merge level (0: the default for nbins); score_cells_per_block:
  * final cells per block of the fused final level (0: the most that fit). */

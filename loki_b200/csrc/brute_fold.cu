@@ -1178,6 +1178,7 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     if (const char* env = std::getenv("LOKI_B200_BF_WARPS")) {
         warps = static_cast<uint32_t>(std::max(1, std::atoi(env)));
     }
+    m_walk_rows = rows;
     require(configure(rows, warps, stages),
             "BruteFold: nbins too large for the shared-memory accumulators");
     m_runs = std::make_unique<RunFold>(freqs, m_seglen, m_nbins, tsamp, t_ref, m_max_batch * m_nseg);
@@ -1303,9 +1304,6 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
         m_map_ev_ptr = nullptr;
         return true;
     }
-    if (stages == run_form_stages()) {
-        stages = kDefaultStages;  // a run-form depth with another form's rows or TMEM warps
-    }
     if ((rows != 1 && rows != 2) || stages < 2 || stages > kMaxStages) {
         return false;
     }
@@ -1368,6 +1366,23 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
     m_map_e_ptr = nullptr;  // the input binding depends on the rows
     m_map_ev_ptr = nullptr;
     return true;
+}
+
+bool BruteFoldDevice::tune(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem) {
+    const bool named = stages == run_form_stages();
+    if (!named && !(stages == 0 && m_use_runs)) {
+        // (the run form's rows and warps with another depth: the depth is what was chosen)
+        const bool present = m_use_runs && rows == m_rows && warps == m_warps;
+        return configure(rows != 0 ? rows : (m_use_runs ? m_walk_rows : m_rows), warps,
+                         stages != 0 ? stages : m_stages, tmem) ||
+               (present && configure(m_walk_rows, 0, stages, tmem));
+    }
+    if (rows != 1 && tmem == 0 && configure(2, warps, run_form_stages())) {
+        return true;
+    }
+    // (a depth that names the run form comes with that form's rows)
+    return configure(rows != 0 ? rows : m_walk_rows, warps, kDefaultStages, tmem) ||
+           (named && configure(m_walk_rows, warps, kDefaultStages, tmem));
 }
 
 uint32_t BruteFoldDevice::max_warps(uint32_t rows, uint32_t stages) const {

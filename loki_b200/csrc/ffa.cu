@@ -377,8 +377,7 @@ void FFAExec::apply_tuning(const lk_tuning& t) {
     require(t.merge_rows_in_flight >= 0 && t.merge_rows_in_flight <= 16,
             "merge rows in flight must lie in [0, 16]");
     if (t.bf_rows != 0 || t.bf_warps != 0 || t.bf_stages != 0 || t.bf_tmem_warps != 0) {
-        require(bf->configure(t.bf_rows != 0 ? t.bf_rows : bf->rows(), t.bf_warps,
-                              t.bf_stages != 0 ? t.bf_stages : bf->stages(), t.bf_tmem_warps),
+        require(bf->tune(t.bf_rows, t.bf_warps, t.bf_stages, t.bf_tmem_warps),
                 "brute-fold launch shape does not fit this plan");
     }
     merge_pb = t.merge_rows_in_flight;

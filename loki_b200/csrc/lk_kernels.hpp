@@ -74,6 +74,10 @@ public:
     // form only). Two rows and stages == run_form_stages() select the
     // run form (brute_fold_runs.cu), the default where it applies.
     bool configure(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem = 0);
+    // A user's launch shape (0: the present value or the rule): the run form
+    // while it is selected or named and takes the shape, else the form that
+    // walks samples, which allows more warps and one row per warp.
+    bool tune(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem);
     uint32_t max_warps(uint32_t rows, uint32_t stages) const;
     // Most tensor-memory warps a block of smem_warps shared-memory warps can add.
     uint32_t max_tmem_warps(uint32_t smem_warps) const;
@@ -111,6 +115,7 @@ private:
     uint64_t m_nwords = 0;
     bool m_wide_bins = false;  // uint16 run bins (nbins > 256)
     uint32_t m_rows = 2;       // rows (E, V) per consumer warp
+    uint32_t m_walk_rows = 2;  // those of the walking form by default
     uint32_t m_warps = 0;      // consumer warps per block
     uint32_t m_stages = 0;     // shared-memory ring depth (32-sample words)
     uint32_t m_tmem = 0;       // consumer warps with tensor-memory sums

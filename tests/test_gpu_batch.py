@@ -215,6 +215,43 @@ def test_autotune_keeps_results(cuda, nbins, lims, storage):
         assert other.tuning[k] == t[k]
 
 
+# nbins -> launch shapes that were taken when the form that walks samples was the
+# only one (the run form allows fewer warps), and shapes no form takes
+SHAPES = {
+    64: ([dict(bf_warps=12), dict(bf_rows=1, bf_warps=19), dict(bf_stages=3), dict(bf_warps=8, bf_tmem_warps=4)],
+         [dict(bf_warps=25), dict(bf_stages=17), dict(bf_rows=3)]),
+    100: ([dict(bf_warps=16), dict(bf_stages=2, bf_warps=10), dict(bf_rows=2, bf_warps=7)],
+          [dict(bf_rows=2, bf_warps=15), dict(bf_warps=17)]),
+    128: ([dict(bf_warps=12), dict(bf_stages=4)],
+          [dict(bf_rows=2, bf_warps=12), dict(bf_warps=12, bf_tmem_warps=4), dict(bf_warps=13)]),
+    1000: ([dict(bf_stages=3), dict(bf_warps=1)], [dict(bf_rows=2, bf_stages=3), dict(bf_warps=14)]),
+}
+
+
+@pytest.mark.parametrize("nbins", sorted(SHAPES))
+def test_launch_shapes_taken_and_refused(cuda, nbins):
+    """Shapes with fields left at 0 (or at the present values) are taken by the
+    run form or by the form that walks samples; results are the same."""
+    from loki_b200.ffa import FFACUDA
+
+    n, lims = 1 << 16, ((20.0, 40.0),)
+    cfg = _cfg(n, nbins, lims, tsamp=64e-6)
+    e, v = series(n, 96)
+    want = FFACUDA(cfg).execute(e, v)
+    taken, refused = SHAPES[nbins]
+    for shape in taken:
+        for base in (False, True):  # on a fresh executor: the fields alone, or changed in its tuning
+            ffa = FFACUDA(cfg)
+            ffa.set_tuning({**ffa.tuning, **shape} if base else shape)
+            assert ffa.tuning["bf_warps"] == shape.get("bf_warps", ffa.tuning["bf_warps"])
+            np.testing.assert_array_equal(ffa.execute(e, v).view(np.uint32), want.view(np.uint32))
+    for shape in refused:
+        ffa = FFACUDA(cfg)
+        with pytest.raises(RuntimeError, match="launch shape"):
+            ffa.set_tuning(shape)
+        np.testing.assert_array_equal(ffa.execute(e, v).view(np.uint32), want.view(np.uint32))
+
+
 def test_autotune_multi_segment_plan(cuda):
     """A plan that stops at several segments (the pruning input) is tuned
     through its brute fold and merges; the fold stays bit-exact."""
