@@ -158,11 +158,14 @@ int lk_plan_resolve_coords(const lk_plan* plan, void* d_coords, uint64_t n_coord
  * LK_FP16: rejected (LK_ERR_UNSUPPORTED): V rows outgrow FP16's range. */
 int lk_ffa_create(const lk_plan* plan, int device, int storage, lk_ffa** out);
 void lk_ffa_destroy(lk_ffa* ffa);
-/* Host check (no device): *fits = 1 when the buffers of an executor of this plan
- * hold every level that a pass over levels 0 .. last stores in them; has_output:
- * the last level goes to a caller's buffer instead. The final level may be
- * larger than all before it, so a pass over every level needs an output. */
-int lk_ffa_levels_fit(const lk_plan* plan, int storage, uint32_t last, int has_output, int* fits);
+/* Host only (no device): the levels stored by the merge launches of a pass over
+ * levels 0 .. last of nbatch series (two levels in one launch store the second;
+ * up to max_levels are written, *n_out is their number). has_output: the last
+ * level goes to a caller's buffer. LK_ERR_INVALID_ARG when a level would not fit
+ * the executor's buffers: the final level may be larger than all before it, so a
+ * pass over every level needs an output. */
+int lk_ffa_level_steps(const lk_plan* plan, int storage, uint64_t nbatch, uint32_t last, int has_output,
+                       uint32_t* levels, uint32_t max_levels, uint32_t* n_out);
 /* Device bytes owned by the executor. */
 int lk_ffa_workspace_bytes(const lk_ffa* ffa, uint64_t* bytes);
 /* Final-level fold, FP32, fold_size floats. Replaces FFACUDA::execute

@@ -188,17 +188,17 @@ void lk_ffa_destroy(lk_ffa* ffa) {
     }
 }
 
-int lk_ffa_levels_fit(const lk_plan* plan, int storage, uint32_t last, int has_output, int* fits) {
+int lk_ffa_level_steps(const lk_plan* plan, int storage, uint64_t nbatch, uint32_t last, int has_output,
+                       uint32_t* levels, uint32_t max_levels, uint32_t* n_out) {
     return guarded([&] {
         need(plan, "plan");
-        need(fits, "fits");
-        const lk::Plan& p = plan->plan;
-        lk::require(last < p.n_levels, "level out of range");
-        *fits = 1;
-        try {
-            lk::ffa_level_steps(p, storage == LK_BF16, last, has_output != 0);
-        } catch (const lk::Error&) {
-            *fits = 0;
+        need(levels, "levels");
+        need(n_out, "n_out");
+        lk::require(last < plan->plan.n_levels, "level out of range");
+        const auto steps = lk::ffa_level_steps(plan->plan, storage == LK_BF16, nbatch, last, has_output != 0);
+        *n_out = static_cast<uint32_t>(steps.size());
+        for (size_t i = 0; i < steps.size() && i < max_levels; ++i) {
+            levels[i] = steps[i].to;
         }
     });
 }

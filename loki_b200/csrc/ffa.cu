@@ -56,16 +56,32 @@ uint64_t ffa_buffer_size(const Plan& plan, bool mixed) {
     return n;
 }
 
-// Levels in pairs, the first alone when their number is odd; levels alternate
-// between the two buffers (a BF16 executor's first output, read from fold0,
-// takes buf[1]).
-std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint32_t last, bool has_output) {
+namespace {
+
+// Whether two levels go in one launch. A pair reads four rows for every row it
+// stores where two launches read two for each level's, so it pays as long as
+// the level between, which it neither stores nor reads back, is not much smaller
+// than its output. us of the pair (of the two launches): equal levels, 25
+// Mfloats of 64 bins 54 (79), 198 of 128 bins 351 (531), 21 of 100 bins 68 (83,
+// BF16 78 (83)); output twice the level between, 43 of 100 bins 132 (112);
+// three times, 74 of 64 bins 135 (128, BF16 124 (106)); four times, 494 of 64
+// bins 746 (669). Small levels save a launch at any ratio: three times, 6.4
+// Mfloats 17 (21), 1.6 9 (15).
+bool pair_levels(uint64_t between, uint64_t out) { return 2 * out <= 3 * between || out <= (8u << 20); }
+
+}  // namespace
+
+// Levels alternate between the two buffers (a BF16 executor's first output, read
+// from fold0, takes buf[1]).
+std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint64_t nbatch, uint32_t last,
+                                       bool has_output) {
     require(last < plan.n_levels, "internal: level out of range");
     const uint64_t have = ffa_buffer_size(plan, mixed);
     std::vector<LevelStep> steps;
     int cur = 0;
     for (uint32_t l = 1; l <= last;) {
-        const uint32_t to = (last - l) % 2 == 1 ? l + 1 : l;
+        const bool two = l < last && pair_levels(nbatch * plan.fold_size(l), nbatch * plan.fold_size(l + 1));
+        const uint32_t to = two ? l + 1 : l;
         const int dest = to == last && has_output ? -1 : 1 - cur;
         require(dest < 0 || plan.fold_size(to) <= have, "a level of this plan needs the caller's output buffer");
         steps.push_back({l - 1, to, dest});
@@ -174,7 +190,7 @@ const void* FFAExec::run_levels(const float* ts_e, const float* ts_v, uint32_t l
                                float* final_out, cudaStream_t s, uint64_t nbatch,
                                bool* last_bf16) {
     require(nbatch >= 1 && nbatch <= max_batch, "nbatch must lie in [1, max_batch]");
-    const std::vector<LevelStep> steps = ffa_level_steps(plan, mixed, last, final_out != nullptr);
+    const std::vector<LevelStep> steps = ffa_level_steps(plan, mixed, nbatch, last, final_out != nullptr);
     const bool taylor = plan.nparams > 1;
     const auto nbins = static_cast<uint32_t>(plan.cfg.nbins);
     // Level l is BF16 when the storage is mixed, l >= 1, and it is not the

@@ -54,10 +54,11 @@ struct LevelStep {
 // Elements (per series) of each of the two intermediate buffers: the largest
 // level before the last (with BF16 storage level 0 has its own).
 uint64_t ffa_buffer_size(const Plan& plan, bool mixed);
-// The merge launches of levels 1 .. last. Fails when a level does not fit the
+// The merge launches of levels 1 .. last of nbatch series. Fails when a level does not fit the
 // buffer it would be stored in (the last level of a plan may be larger than
 // every level before it and then needs the caller's output).
-std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint32_t last, bool has_output);
+std::vector<LevelStep> ffa_level_steps(const Plan& plan, bool mixed, uint64_t nbatch, uint32_t last,
+                                       bool has_output);
 
 struct FFAExec {
     Plan plan;

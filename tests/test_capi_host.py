@@ -150,7 +150,6 @@ def test_params_dict_and_fold_shapes():
 def test_last_level_larger_than_the_buffers(bf16, accel, bseg):
     """A plan that stops at several segments and whose last level is its
     largest: only the caller's output holds that level."""
-    from loki_b200 import _capi as C
     from loki_b200.configs import PulsarSearchConfig
     from loki_b200.plans import FFAPlanTime
 
@@ -159,8 +158,46 @@ def test_last_level_larger_than_the_buffers(bf16, accel, bseg):
     plan = FFAPlanTime(cfg)
     sizes = [int(n) * int(c) * 64 for n, c in zip(plan.nsegments, plan.ncoords)]
     assert plan.nsegments[-1] > 1 and sizes[-1] > 2 * max(sizes[:-1])
-    fits = ctypes.c_int(-1)
     for last in range(plan.n_levels):
         for has_output in (0, 1):
-            C.check(C.lib().lk_ffa_levels_fit(plan._handle, 1 if bf16 else 0, last, has_output, ctypes.byref(fits)))
-            assert fits.value == (1 if has_output or last + 1 < plan.n_levels else 0)
+            steps = _level_steps(plan, bf16, 1, last, has_output)
+            assert (steps is not None) == bool(has_output or last + 1 < plan.n_levels)
+
+
+# (plan, series of a batch, last level, levels stored): pairs while the output is
+# at most 1.5 times the level between or at most 8 Mi floats, else one at a time
+STEPS = {
+    "equal_even": ((2**21, 64e-6, 128, 1.0, [[5.0, 50.0]], None), 1, 6, [2, 4, 6]),
+    "equal_odd": ((2**21, 64e-6, 128, 1.0, [[5.0, 50.0]], None), 1, 7, [2, 4, 6, 7]),
+    "last_three_times": ((2**22, 64e-6, 64, 2.0, [[-200.0, 200.0], [5.0, 50.0]], None), 1, 7, [2, 4, 6, 7]),
+    "growing": ((2**18, 1e-3, 32, 1.0, [[-20000.0, 20000.0], [5.0, 8.0]], 2**17), 1, 7, [2, 4, 6, 7]),
+    "growing_batch": ((2**18, 1e-3, 32, 1.0, [[-20000.0, 20000.0], [5.0, 8.0]], 2**17), 8, 7, [2, 4, 5, 6, 7]),
+    "one_level": ((2**18, 1e-3, 32, 1.0, [[-20000.0, 20000.0], [5.0, 8.0]], 2**17), 8, 1, [1]),
+    "none": ((2**18, 1e-3, 32, 1.0, [[-20000.0, 20000.0], [5.0, 8.0]], 2**17), 8, 0, []),
+}
+
+
+def _level_steps(plan, bf16, nbatch, last, has_output):
+    """Levels stored by the merge launches, or None where one does not fit."""
+    from loki_b200 import _capi as C
+
+    levels = (ctypes.c_uint32 * 64)()
+    n = ctypes.c_uint32()
+    rc = C.lib().lk_ffa_level_steps(plan._handle, 1 if bf16 else 0, nbatch, last, has_output, levels, 64,
+                                    ctypes.byref(n))
+    if rc == C.LK_ERR_INVALID_ARG:
+        return None
+    C.check(rc)
+    return list(levels[: n.value])
+
+
+@pytest.mark.parametrize("name", sorted(STEPS))
+def test_merge_launches(name):
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.plans import FFAPlanTime
+
+    (nsamps, tsamp, nbins, eta, lims, bseg_ffa), nbatch, last, want = STEPS[name]
+    cfg = PulsarSearchConfig(nsamps, tsamp, nbins, eta, np.array(lims), use_fourier=False, bseg_ffa=bseg_ffa)
+    plan = FFAPlanTime(cfg)
+    for bf16 in (False, True):
+        assert _level_steps(plan, bf16, nbatch, last, 1) == want
