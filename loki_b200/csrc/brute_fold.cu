@@ -1377,12 +1377,12 @@ bool BruteFoldDevice::tune(uint32_t rows, uint32_t warps, uint32_t stages, uint3
                          stages != 0 ? stages : m_stages, tmem) ||
                (present && configure(m_walk_rows, 0, stages, tmem));
     }
-    if (rows != 1 && tmem == 0 && configure(2, warps, run_form_stages())) {
+    if ((rows == 0 || rows == 2) && tmem == 0 && configure(2, warps, run_form_stages())) {
         return true;
     }
     // (a depth that names the run form comes with that form's rows)
     return configure(rows != 0 ? rows : m_walk_rows, warps, kDefaultStages, tmem) ||
-           (named && configure(m_walk_rows, warps, kDefaultStages, tmem));
+           (named && rows == 2 && configure(m_walk_rows, warps, kDefaultStages, tmem));
 }
 
 uint32_t BruteFoldDevice::max_warps(uint32_t rows, uint32_t stages) const {
