@@ -1181,6 +1181,7 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
     m_walk_rows = rows;
     require(configure(rows, warps, stages),
             "BruteFold: nbins too large for the shared-memory accumulators");
+    m_walk_warps = m_warps;
     m_runs = std::make_unique<RunFold>(freqs, m_seglen, m_nbins, tsamp, t_ref, m_max_batch * m_nseg);
     if (!m_runs->ok()) {
         m_runs.reset();
@@ -1369,20 +1370,18 @@ bool BruteFoldDevice::configure(uint32_t rows, uint32_t warps, uint32_t stages, 
 }
 
 bool BruteFoldDevice::tune(uint32_t rows, uint32_t warps, uint32_t stages, uint32_t tmem) {
-    const bool named = stages == run_form_stages();
-    if (!named && !(stages == 0 && m_use_runs)) {
-        // (the run form's rows and warps with another depth: the depth is what was chosen)
-        const bool present = m_use_runs && rows == m_rows && warps == m_warps;
-        return configure(rows != 0 ? rows : (m_use_runs ? m_walk_rows : m_rows), warps,
-                         stages != 0 ? stages : m_stages, tmem) ||
-               (present && configure(m_walk_rows, 0, stages, tmem));
-    }
-    if ((rows == 0 || rows == 2) && tmem == 0 && configure(2, warps, run_form_stages())) {
+    const bool runs = stages == run_form_stages() || (stages == 0 && m_use_runs);
+    if (runs && (rows == 0 || rows == 2) && tmem == 0 && configure(2, warps, run_form_stages())) {
         return true;
     }
-    // (a depth that names the run form comes with that form's rows)
-    return configure(rows != 0 ? rows : m_walk_rows, warps, kDefaultStages, tmem) ||
-           (named && rows == 2 && configure(m_walk_rows, warps, kDefaultStages, tmem));
+    const uint32_t depth = runs ? kDefaultStages : (stages != 0 ? stages : m_stages);
+    if (configure(rows != 0 ? rows : (m_use_runs ? m_walk_rows : m_rows), warps, depth, tmem)) {
+        return true;
+    }
+    // The run form's present values with one of them changed: the others are
+    // that form's, not a choice, and stand for the walking form's own.
+    return m_use_runs && rows != 0 && warps != 0 && stages != 0 &&
+           configure(rows == m_rows ? m_walk_rows : rows, warps == m_warps ? m_walk_warps : warps, depth, tmem);
 }
 
 uint32_t BruteFoldDevice::max_warps(uint32_t rows, uint32_t stages) const {

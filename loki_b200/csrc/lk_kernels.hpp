@@ -115,7 +115,8 @@ private:
     uint64_t m_nwords = 0;
     bool m_wide_bins = false;  // uint16 run bins (nbins > 256)
     uint32_t m_rows = 2;       // rows (E, V) per consumer warp
-    uint32_t m_walk_rows = 2;  // those of the walking form by default
+    uint32_t m_walk_rows = 2;  // rows and warps of the walking form by default
+    uint32_t m_walk_warps = 0;
     uint32_t m_warps = 0;      // consumer warps per block
     uint32_t m_stages = 0;     // shared-memory ring depth (32-sample words)
     uint32_t m_tmem = 0;       // consumer warps with tensor-memory sums
