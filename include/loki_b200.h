@@ -448,6 +448,11 @@ void lk_brute_fold_destroy(lk_brute_fold* bf);
 /* d_fold: [nsamps/segment_len, nfreqs, 2, nbins] FP32. */
 int lk_brute_fold_execute(lk_brute_fold* bf, const float* d_ts_e, const float* d_ts_v,
                           float* d_fold, lk_stream_t stream);
+/* Host only (no device): *run_form = 1 where the run form is the brute fold's
+ * default for max_batch series of nsamps samples; *bytes: its transposed series
+ * (0 where it does not take the frequencies at all). */
+int lk_brute_fold_form(const double* freqs, uint64_t nfreqs, uint64_t segment_len, uint64_t nbins, uint64_t nsamps,
+                       double tsamp, double t_ref, uint64_t max_batch, int* run_form, uint64_t* bytes);
 /* Host replay (no device) of the run tables of the brute fold's run form
  * over one segment `ts` [segment_len] of one row, every read checked against
  * the padded segment: fold [nfreqs * nbins]; *applies = 0 (fold untouched)

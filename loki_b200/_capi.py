@@ -195,6 +195,7 @@ SIGNATURES = [
     ("lk_brute_fold_create", i32, [vp, u64, u64, u64, u64, f64, f64, i32, vp]),
     ("lk_brute_fold_destroy", None, [vp]),
     ("lk_brute_fold_execute", i32, [vp, vp, vp, vp, vp]),
+    ("lk_brute_fold_form", i32, [vp, u64, u64, u64, u64, f64, f64, u64, vp, vp]),
     ("lk_brute_fold_replay", i32, [vp, u64, u64, u64, f64, f64, vp, vp, vp]),
     ("lk_box_width_trials", i32, [u64, f64, f64, vp, u32, vp]),
     ("lk_snr_boxcar_3d", i32, [vp, u64, u32, vp, u32, i32, vp, vp]),

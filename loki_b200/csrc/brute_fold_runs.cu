@@ -712,6 +712,39 @@ RunTables build_tables(const std::vector<double>& freqs, uint64_t segment_len, u
 
 }  // namespace
 
+namespace {
+
+uint64_t transposed_bytes(uint64_t max_rows, uint32_t nstages) {
+    return (max_rows + 31) / 32 * nstages * kStageBytes;
+}
+
+// Whether the run form is taken for a call's segments. Speed: every block streams
+// the padding too, four runs and more on both sides. Against the form that walks
+// samples (times as fast, unit variances / others), 2^20 and 2^22 samples, 48 and
+// 96 frequencies, 16 to 128 bins: segments of 2048 samples and more padded to
+// less than twice their length 1.1 to 4.3 / 1.0 to 2.5, to 4.5 times 0.7 to 1.0;
+// segments of 256 to 1024 samples padded to at most 1.5 times 1.0 to 2.3 / 0.82 to
+// 1.7 (below 1 where bins are skipped or hold 9 and more samples), to 3.7 and
+// 10 times 0.6 to 1.0 / 0.35 to 0.7; of 64 and 16 samples, padded to 2 and 6
+// times and more, 0.8 to 1.2 / 0.7 to 1.2. Memory: 32 segments' worth for each group even
+// where the call has fewer (2 to 4.5 times as fast there all the same), so at
+// most twice the series' (e, v) pairs or 1 GiB.
+bool run_form_pays(uint64_t segment_len, uint32_t nstages, uint64_t max_rows) {
+    const uint64_t padded = static_cast<uint64_t>(nstages) * kStageLen;
+    const uint64_t pairs = max_rows * segment_len * sizeof(float2);
+    return (segment_len >= 2048 ? padded <= 2 * segment_len : 2 * padded <= 3 * segment_len) &&
+           transposed_bytes(max_rows, nstages) <= std::max<uint64_t>(2 * pairs, 1ull << 30);
+}
+
+}  // namespace
+
+bool run_form_applies(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp,
+                      double t_ref, uint64_t max_rows, uint64_t* bytes) {
+    const RunTables tb = build_tables(freqs, segment_len, static_cast<uint32_t>(nbins), tsamp, t_ref);
+    *bytes = tb.ok ? transposed_bytes(max_rows, tb.nstages) : 0;
+    return tb.ok && run_form_pays(segment_len, tb.nstages, max_rows);
+}
+
 RunFold::RunFold(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref,
                  uint64_t max_rows)
     : m_nfreq(static_cast<uint32_t>(freqs.size())),
@@ -719,7 +752,7 @@ RunFold::RunFold(const std::vector<double>& freqs, uint64_t segment_len, uint64_
       m_seglen(static_cast<uint32_t>(segment_len)),
       m_max_rows(max_rows) {
     const RunTables tb = build_tables(freqs, segment_len, m_nbins, tsamp, t_ref);
-    if (!tb.ok) {
+    if (!tb.ok || !run_form_pays(segment_len, tb.nstages, max_rows)) {
         return;
     }
     m_nranges = tb.nranges;
@@ -855,7 +888,7 @@ void RunFold::reserve() {
         return;
     }
     m_varied.alloc((m_max_rows + 63) / 64 * sizeof(uint32_t));
-    m_evt.alloc((m_max_rows + 31) / 32 * m_nstages * kStageBytes);
+    m_evt.alloc(transposed_bytes(m_max_rows, m_nstages));
     // the zeros before and after each segment stay; the samples between them
     // are written by every call, on any stream
     LK_CUDA(cudaMemsetAsync(m_evt.ptr, 0, m_evt.bytes, nullptr));

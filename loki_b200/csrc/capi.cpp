@@ -779,6 +779,21 @@ int lk_brute_fold_replay(const double* freqs, uint64_t nfreqs, uint64_t segment_
     });
 }
 
+int lk_brute_fold_form(const double* freqs, uint64_t nfreqs, uint64_t segment_len, uint64_t nbins, uint64_t nsamps,
+                       double tsamp, double t_ref, uint64_t max_batch, int* run_form, uint64_t* bytes) {
+    return guarded([&] {
+        need(freqs, "freqs");
+        need(run_form, "run_form");
+        need(bytes, "bytes");
+        lk::require(segment_len > 0 && nbins >= 1 && nbins <= 65535, "BruteFold: bad segment length or nbins");
+        lk::require(nfreqs >= 1 && std::all_of(freqs, freqs + nfreqs, [](double f) { return f >= 0.0; }),
+                    "Frequency must be positive");
+        const std::vector<double> f(freqs, freqs + nfreqs);
+        const uint64_t rows = max_batch * (nsamps / segment_len);
+        *run_form = lk::run_form_applies(f, segment_len, nbins, tsamp, t_ref, rows, bytes) ? 1 : 0;
+    });
+}
+
 int lk_brute_fold_execute(lk_brute_fold* bf, const float* d_ts_e, const float* d_ts_v,
                           float* d_fold, lk_stream_t stream) {
     return guarded([&] {

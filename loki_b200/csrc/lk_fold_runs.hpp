@@ -25,10 +25,15 @@ void fold_runs(double freq, uint64_t segment_len, uint64_t nbins, double tsamp, 
 bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp,
                      double t_ref, const float* ts, float* fold);
 
+// Whether the run form is the default for calls of up to max_rows segments;
+// bytes: of its transposed series.
+bool run_form_applies(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp,
+                      double t_ref, uint64_t max_rows, uint64_t* bytes);
+
 class RunFold {
 public:
     // Builds the tables; ok() is false when a frequency's runs do not have
-    // the form the kernel takes (see brute_fold_runs.cu).
+    // the form the kernel takes, or where it does not pay (brute_fold_runs.cu).
     // max_rows: most segments of a call.
     RunFold(const std::vector<double>& freqs, uint64_t segment_len, uint64_t nbins, double tsamp, double t_ref,
             uint64_t max_rows);

@@ -57,3 +57,37 @@ def test_left_to_the_other_form():
     for nbins, seglen, tsamp, f in ((64, 1024, 1e-3, 900.0), (2, 1 << 16, 64e-6, 0.9)):
         applies, _ = _replay(np.array([f]), seglen, nbins, tsamp, 0.0, np.ones(seglen, np.float32))
         assert applies == 0
+
+
+# (segment_len, nsamps, samples per bin, nbins, batch, run form): segments with
+# little padding, short ones padded to more than 1.5 times, long ones to more than
+# twice; few segments below and above 1 GiB
+FORMS = {
+    "plan": (16384, 1 << 22, 9.0, 64, 1, True),
+    "short_segments": (1024, 1 << 16, 6.0, 32, 1, True),
+    "samples_256": (256, 1 << 20, 2.0, 64, 1, True),
+    "samples_4": (4, 1 << 16, 0.8, 16, 1, False),
+    "samples_64": (64, 1 << 20, 3.0, 64, 1, False),
+    "samples_256_at_1.5": (256, 1 << 20, 9.0, 16, 1, True),
+    "samples_256_padded": (256, 1 << 20, 20.0, 16, 1, False),
+    "samples_1024_padded": (1024, 1 << 20, 60.0, 16, 1, False),
+    "samples_4096": (4096, 1 << 20, 300.0, 4, 1, True),
+    "samples_4096_padded": (4096, 1 << 20, 1500.0, 2, 1, False),
+    "one_segment": (1 << 20, 1 << 20, 9.0, 64, 1, True),
+    "one_long_segment": (1 << 23, 1 << 23, 9.0, 64, 1, False),
+    "one_long_segment_of_32": (1 << 23, 1 << 23, 9.0, 64, 32, True),
+}
+
+
+@pytest.mark.parametrize("name", sorted(FORMS))
+def test_form_and_its_memory(name):
+    from loki_b200 import _capi as C
+
+    seglen, nsamps, samples, nbins, batch, want = FORMS[name]
+    f = np.array([1.0 / (samples * 64e-6 * nbins)])
+    form, size = ctypes.c_int(-1), ctypes.c_uint64()
+    C.check(C.lib().lk_brute_fold_form(f.ctypes.data, 1, seglen, nbins, nsamps, 64e-6, 0.0, batch,
+                                       ctypes.byref(form), ctypes.byref(size)))
+    assert form.value == (1 if want else 0)
+    if want:  # at most twice the series' pairs, or 1 GiB
+        assert 0 < size.value <= max(2 * 8 * nsamps * batch, 1 << 30)
