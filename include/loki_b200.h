@@ -378,9 +378,13 @@ int lk_sweep_results(const lk_sweep* sw, double* params, float* scores, uint64_t
  * Fields at 0 keep the present value or the rule; while the run form is in use
  * or named, a shape that it does not take (one row, more warps, TMEM warps) goes
  * to the form that walks samples;
- * merge_rows_in_flight: output rows per warp whose loads are issued
- * together in a merge level (0: the default for nbins); score_cells_per_block:
- * final cells per block of the fused final level (0: the most that fit). */
+ * merge_rows_in_flight: output rows per warp whose loads are issued together in
+ * a merge level that has a launch of its own (0: the default for nbins; levels
+ * that go two in a launch have no such choice); score_cells_per_block: final
+ * cells per block of the generic final level, up to 128 bins (32 and more), or
+ * 0 (the kernel for the plan's bins and widths) or 1 (the same without its table
+ * of 1 / sqrt(V), 32, 64 and 128 bins); without effect above 128 bins. The
+ * autotuner leaves a field without a choice at 0. */
 typedef struct lk_tuning {
     uint32_t bf_rows;
     uint32_t bf_warps;

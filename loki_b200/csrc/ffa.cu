@@ -158,9 +158,11 @@ FFAExec::FFAExec(const Plan& p, int device, int storage, uint64_t max_batch_)
     if (plan.nsegments[plan.n_levels - 1] == 1 &&
         make_mask_score_params(sp, static_cast<uint32_t>(plan.cfg.nbins), &mp, true)) {
         wm = true;
-        normtab.alloc(sizeof(float) * kNormTableSize);
-        norm_table_fill(normtab.as<float>(), nullptr);
-        LK_CUDA(cudaDeviceSynchronize());
+        if (final_level_uses_table(static_cast<uint32_t>(plan.cfg.nbins))) {
+            normtab.alloc(sizeof(float) * kNormTableSize);
+            norm_table_fill(normtab.as<float>(), nullptr);
+            LK_CUDA(cudaDeviceSynchronize());
+        }
     }
 }
 
@@ -278,7 +280,7 @@ void FFAExec::scores_impl(const float* ts_e, const float* ts_v, float* d_scores,
                              plan.ncoords[L - 1] / n_inner, plan.ncoords[L - 2],
                              static_cast<uint32_t>(plan.cfg.nbins), mp, LK_SCORE_PER_WIDTH,
                              d_scores, s, nbatch, in_bf16, d_cmax, normtab.as<float>(), count_thr,
-                             d_counts, score_cells == 0);
+                             d_counts, score_cells == 0 && normtab.ptr != nullptr);
     } else {
         require(d_counts == nullptr, "internal: block counts need the masked final level");
         merge_score_level(in, level_coords(L - 1), plan.nparams > 1, n_inner,
@@ -544,8 +546,14 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
         }
         float merge_best = INFINITY;
         int bpb = 0;
-        // levels 1 .. L-2 are plain merges when scoring, 1 .. L-1 otherwise
-        if (plan.n_levels > (scoring ? 2u : 1u)) {
+        // Levels 1 .. L-2 are plain merges when scoring, 1 .. L-1 otherwise; the
+        // rows in flight are a choice where some level goes alone.
+        const std::vector<LevelStep> steps =
+            ffa_level_steps(plan, mixed, 1, plan.n_levels - (scoring ? 2 : 1), !scoring);
+        if (std::none_of(steps.begin(), steps.end(), [](const LevelStep& st) { return st.to == st.from + 1; })) {
+            pbs = {0};
+        }
+        if (!steps.empty()) {
             for (int pb : pbs) {
                 merge_pb = pb;
                 const float ms = time_stages({LK_STAGE_MERGE});
@@ -558,23 +566,26 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
             merge_best = 0.0f;
         }
         merge_pb = bpb;
-        // 3. fused final level: cells per block
+        // 3. fused final level: the masked kernel (final_level.cu) with and
+        // without its table, and the generic kernel's cells per block (above
+        // 128 bins a kernel without such a choice)
         const uint32_t rs = sc::row_stride(nb, sp.wmax);
         const uint32_t tmax = sc::profiles_per_block(rs);
         float score_best = scoring ? INFINITY : 0.0f;
         uint32_t bcells = 0;
-        if (scoring && wm) {
-            // masked final level (final_level.cu), with and without the table
-            for (uint32_t v : {0u, 1u}) {
-                score_cells = v;
-                const float ms = time_stages({LK_STAGE_MERGE_SCORE});
-                if (ms < score_best) {
-                    score_best = ms;
-                    bcells = v;
-                }
+        std::vector<uint32_t> choices;
+        if (scoring) {
+            if (wm || nb > 128) {
+                choices.push_back(0);
+            }
+            if (normtab.ptr != nullptr) {
+                choices.push_back(1);
+            }
+            for (uint32_t cells = 32; nb <= 128 && cells <= tmax; cells += 32) {
+                choices.push_back(cells);
             }
         }
-        for (uint32_t cells = 32; scoring && cells <= tmax; cells += 32) {
+        for (const uint32_t cells : choices) {
             score_cells = cells;
             const float ms = time_stages({LK_STAGE_MERGE_SCORE});
             if (ms < score_best) {

@@ -519,7 +519,7 @@ void norm_table_fill(float* d_tab, cudaStream_t s) {
 }
 
 bool make_mask_score_params(const ScoreParams& sp, uint32_t nbins, MaskScoreParams* mp, bool any_nbins) {
-    if (any_nbins ? nbins > 128 : nbins != 32 && nbins != 64 && nbins != 128) {
+    if (any_nbins ? nbins > 128 : !final_level_uses_table(nbins)) {
         return false;
     }
     MaskScoreParams m{};
@@ -540,6 +540,8 @@ bool make_mask_score_params(const ScoreParams& sp, uint32_t nbins, MaskScorePara
     *mp = m;
     return true;
 }
+
+bool final_level_uses_table(uint32_t nbins) { return nbins == 32 || nbins == 64 || nbins == 128; }
 
 uint32_t final_level_cells_per_block() { return 128; }
 

@@ -102,8 +102,8 @@ struct FFAExec {
     // up new lengths written into the same array.
     const uint64_t* batch_lens = nullptr;
     // Tuned launch shapes (0: defaults); see autotune.
-    int merge_pb = 0;            // merge: output rows per warp in flight
-    uint32_t score_cells = 0;    // final level + score: cells per block
+    int merge_pb = 0;            // merge levels alone in a launch: output rows per warp in flight
+    uint32_t score_cells = 0;    // final level + score: kernel (0, 1) or the generic one's cells per block
     lk_tuning tuning{};          // last autotune result / applied shapes
 
     // Times launch-shape candidates of the brute fold (rows per warp,

@@ -187,6 +187,8 @@ struct MaskScoreParams {
 // wider than 32 bins).
 bool make_mask_score_params(const ScoreParams& sp, uint32_t nbins, MaskScoreParams* mp,
                             bool any_nbins = false);
+// Whether the masked kernel of nbins can read 1 / sqrt(V) from the table.
+bool final_level_uses_table(uint32_t nbins);
 uint32_t final_level_cells_per_block();
 // Blocks (count slots) of one final-level launch.
 uint64_t final_level_blocks(uint64_t n_inner, uint64_t n_outer, uint64_t nbatch);

@@ -215,6 +215,33 @@ def test_autotune_keeps_results(cuda, nbins, lims, storage):
         assert other.tuning[k] == t[k]
 
 
+@pytest.mark.parametrize("nbins, nsamps", [(64, 1 << 16), (64, 1 << 17), (256, 1 << 16), (256, 1 << 17)])
+def test_autotune_times_only_real_choices(cuda, nbins, nsamps):
+    """Fields without a choice cost no candidate and stay 0: the rows in flight
+    where every merge level goes in a pair, the cells per block above 128 bins."""
+    from loki_b200.ffa import FFACUDA
+
+    cfg = _cfg(nsamps, nbins, ((20.0, 40.0),), tsamp=64e-6)
+    ffa = FFACUDA(cfg)
+    alone = (ffa.plan.n_levels - 2) % 2 == 1  # the last merge before the final level
+    assert alone == (nsamps == 1 << 17)
+    e, v = series(nsamps, 97)
+    want = ffa.scores(e, v)
+    run_warps = 0
+    for w in range(4, 21):
+        try:
+            ffa.set_tuning(dict(bf_rows=2, bf_stages=32, bf_warps=w))
+            run_warps += ffa.tuning["bf_stages"] == 32
+        except RuntimeError:
+            pass
+    t = ffa.autotune(e, v, reps=1)
+    assert t["bf_stages"] == 32 and run_warps > 1
+    assert t["merge_rows_in_flight"] in ((2, 4, 8) if alone and nbins == 64 else (0,))
+    if nbins > 128:
+        assert t["score_cells_per_block"] == 0 and t["candidates"] == run_warps + 2
+    np.testing.assert_array_equal(ffa.scores(e, v).view(np.uint32), want.view(np.uint32))
+
+
 # nbins -> launch shapes that were taken when the form that walks samples was the
 # only one (the run form allows fewer warps), and shapes no form takes
 SHAPES = {
