@@ -195,15 +195,24 @@ def smem_peak_gbs(device_index, clk):
     return 128 * props.multi_processor_count * mhz * 1e6 / 1e9
 
 
+def fold_reads(params, ffa):
+    """4-byte shared-memory reads of the samples in the last search's level-0
+    fold: one per sample and level-0 frequency for each row folded. Groups of
+    segments with unit variances fold E alone, others E and V."""
+    checked, varied = ffa.unit_groups()
+    rows = 2.0 if checked == 0 else 1.0 + varied / checked
+    return int(rows * params["nsamps"] * int(ffa.plan.param_counts[0][-1]))
+
+
 def stage_roofline(stage_ms, stage_bytes, steps, clk, device_index, brute_adds):
     """Roofline object of the dominant stage.
 
     HBM-bound stages (merges, merge+score, compaction) report algorithmic HBM
     bytes per launch / average launch time against the measured copy peak.
     The level-0 brute fold reads little HBM data: its bound is shared memory
-    (one 4-byte read per sample x level-0 frequency x row from the staged
-    series tile, brute_adds = those reads), so it is reported as "smem"
-    against the nominal shared-memory bandwidth, with its HBM fraction kept as
+    (one 4-byte read per sample x level-0 frequency x row that is folded, from
+    the staged series tile, brute_adds = those reads, see fold_reads), so it is
+    reported as "smem" against the nominal shared-memory bandwidth, with its HBM fraction kept as
     a second field. Every merge level's HBM fraction is listed too."""
     dom = max(stage_ms, key=stage_ms.get)
     dom_ms = stage_ms[dom] / steps
@@ -572,7 +581,7 @@ def run_ours(args, rank, world, local_rank):
 
     # roofline of the dominant stage
     roofline = stage_roofline(stage_ms, stage_bytes, args.steps, clk, local_rank,
-                              2 * params["nsamps"] * int(ffa.plan.param_counts[0][-1]))
+                              fold_reads(params, ffa))
     stages = {k: {"avg_ms": stage_ms[k] / args.steps, "bytes": stage_bytes[k],
                   "gbs": stage_bytes[k] / (stage_ms[k] / args.steps / 1e3) / 1e9}
               for k in sorted(stage_ms, key=stage_ms.get, reverse=True)}

@@ -217,7 +217,7 @@ def run_freq(args, rank, world, local_rank):
     if rank == 0 and not args.no_parity:
         parity = B.candidate_parity(params, ts_e, ts_v, idx[:ncand].cpu().numpy(), snr[:ncand].cpu().numpy())
     roof = B.stage_roofline({k: v[0] for k, v in prof.items()}, {k: v[1] for k, v in prof.items()}, 1, clk,
-                            local_rank, 2 * params["nsamps"] * int(ffa.plan.param_counts[0][-1]))
+                            local_rank, B.fold_reads(params, ffa))
     status = 0
     if rank == 0:
         B.emit(_line(args, world, "freq_sweep_2^21x64us_nbins128", value, ms,

@@ -166,6 +166,10 @@ void lk_ffa_destroy(lk_ffa* ffa);
  * pass over every level needs an output. */
 int lk_ffa_level_steps(const lk_plan* plan, int storage, uint64_t nbatch, uint32_t last, int has_output,
                        uint32_t* levels, uint32_t max_levels, uint32_t* n_out);
+/* How the last call folded: groups of 64 segments whose variances were checked
+ * (0: none, every segment folded E and V; synchronises the stream) and those of
+ * them that have other variances than 1. The rest folded E alone. */
+int lk_ffa_unit_groups(const lk_ffa* ffa, lk_stream_t stream, uint64_t* checked, uint64_t* varied);
 /* Device bytes owned by the executor. */
 int lk_ffa_workspace_bytes(const lk_ffa* ffa, uint64_t* bytes);
 /* Final-level fold, FP32, fold_size floats. Replaces FFACUDA::execute

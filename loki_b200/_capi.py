@@ -151,6 +151,7 @@ SIGNATURES = [
     ("lk_ffa_create", i32, [vp, i32, i32, vp]),
     ("lk_ffa_destroy", None, [vp]),
     ("lk_ffa_level_steps", i32, [vp, i32, u64, u32, i32, vp, u32, vp]),
+    ("lk_ffa_unit_groups", i32, [vp, vp, vp, vp]),
     ("lk_ffa_workspace_bytes", i32, [vp, vp]),
     ("lk_ffa_execute", i32, [vp, vp, vp, vp, u64, vp]),
     ("lk_ffa_scores", i32, [vp, vp, vp, vp, u64, vp]),

@@ -1398,6 +1398,13 @@ uint64_t BruteFoldDevice::device_bytes() const {
            m_ev.bytes + m_seq.bytes + m_groups.bytes + (m_runs ? m_runs->device_bytes() : 0);
 }
 
+void BruteFoldDevice::unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const {
+    *checked = *varied = 0;
+    if (m_use_runs) {
+        m_runs->unit_groups(checked, varied, s);
+    }
+}
+
 // The TMA maps read the series in place; a base address that is not 16-byte
 // aligned (a TMA requirement) is first copied into an aligned staging buffer.
 // A batch of nbatch series stored back to back is folded as one series of

@@ -903,6 +903,7 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
     require(ngrp * tiles <= 0x7fffffffULL && nrows <= m_max_rows, "BruteFold: too many segments");
     const bool vec4 = (reinterpret_cast<uintptr_t>(d_e) % 16 == 0) && (reinterpret_cast<uintptr_t>(d_v) % 16 == 0);
     m_unit = pairs_e(nrows, warps);
+    m_rows = nrows;
     const uint64_t g64 = (nrows + 63) / 64;
     if (m_unit) {
         LK_CUDA(cudaMemsetAsync(m_varied.ptr, 0, g64 * sizeof(uint32_t), s));
@@ -915,6 +916,14 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
                                              m_pad, static_cast<uint32_t>(qlen), vec4, groups, ngroups,
                                              m_unit ? m_varied.as<uint32_t>() : nullptr);
     LK_CUDA(cudaGetLastError());
+}
+
+void RunFold::unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const {
+    std::vector<uint32_t> flags(m_unit ? (m_rows + 63) / 64 : 0);
+    LK_CUDA(cudaMemcpyAsync(flags.data(), m_varied.ptr, flags.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    LK_CUDA(cudaStreamSynchronize(s));
+    *checked = flags.size();
+    *varied = static_cast<uint64_t>(std::count_if(flags.begin(), flags.end(), [](uint32_t x) { return x != 0; }));
 }
 
 void RunFold::fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t* groups,

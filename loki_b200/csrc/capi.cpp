@@ -203,6 +203,16 @@ int lk_ffa_level_steps(const lk_plan* plan, int storage, uint64_t nbatch, uint32
     });
 }
 
+int lk_ffa_unit_groups(const lk_ffa* ffa, lk_stream_t stream, uint64_t* checked, uint64_t* varied) {
+    return guarded([&] {
+        need(ffa, "ffa");
+        need(checked, "checked");
+        need(varied, "varied");
+        lk::DeviceGuard g(ffa->exec->device);
+        ffa->exec->bf->unit_groups(checked, varied, static_cast<cudaStream_t>(stream));
+    });
+}
+
 int lk_ffa_workspace_bytes(const lk_ffa* ffa, uint64_t* bytes) {
     return guarded([&] {
         need(ffa, "ffa");

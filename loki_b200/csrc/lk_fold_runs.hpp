@@ -59,6 +59,10 @@ public:
                    const uint32_t* ngroups, cudaStream_t s);
     void fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t* groups,
               const uint32_t* ngroups, uint32_t* d_status, cudaStream_t s) const;
+    // Groups of 64 segments whose variances the last transpose() checked (0: not
+    // checked, both rows folded) and those found with other variances than 1
+    // (synchronises s).
+    void unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const;
     uint64_t device_bytes() const {
         return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes + m_varied.bytes;
     }
@@ -67,6 +71,7 @@ private:
     bool pairs_e(uint64_t nrows, uint32_t warps) const;
     bool m_ok = false;
     bool m_unit = false;  // the transposed rows were checked for unit variances
+    uint64_t m_rows = 0;  // of the last transpose()
     uint32_t m_nfreq, m_nbins, m_seglen;
     uint32_t m_nranges = 1, m_range = 0;  // bin ranges per frequency, bins per range
     uint32_t m_pad = 0;                   // zero samples before each segment

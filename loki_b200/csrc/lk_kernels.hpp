@@ -98,6 +98,9 @@ public:
     uint64_t nfreq() const { return m_nfreq; }
     uint64_t fold_size() const { return m_nseg * m_nfreq * 2 * m_nbins; }
     uint64_t device_bytes() const;
+    // Groups of 64 segments whose variances the last fold checked, and those
+    // with others than 1 (see RunFold; 0 in the forms without the check).
+    void unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const;
 
 private:
     // Builds the segment-group table of the bound batch on s when d_lens

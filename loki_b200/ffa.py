@@ -242,6 +242,15 @@ class FFACUDA:
             for i in range(min(n.value, 128))
         ]
 
+    def unit_groups(self) -> tuple[int, int]:
+        """(checked, varied) of the last call: groups of 64 level-0 segments
+        whose variances were checked (0: every segment folded E and V) and those
+        with other variances than 1; the rest folded E alone."""
+        checked, varied = ctypes.c_uint64(), ctypes.c_uint64()
+        C.check(C.lib().lk_ffa_unit_groups(self._h, D.stream_ptr(self._device), ctypes.byref(checked),
+                                           ctypes.byref(varied)))
+        return int(checked.value), int(varied.value)
+
     def status(self) -> int:
         st = ctypes.c_uint32()
         C.check(C.lib().lk_ffa_status(self._h, D.stream_ptr(self._device), ctypes.byref(st)))

@@ -43,3 +43,26 @@ def test_other_configs_summary(monkeypatch):
         else:
             assert rec["rc"] == 0 and rec["workload"] == name + "_w"
             assert rec["value"] == 2.0 and rec["e2e"] == 1.5 and rec["parity"]["candidates_match"]
+
+
+def test_fold_reads_count_the_rows_folded():
+    """The fold's roofline credits E alone for groups with unit variances."""
+
+    class Plan:
+        param_counts = [[1, 755]]
+
+    class Ffa:
+        plan = Plan()
+
+        def __init__(self, checked, varied):
+            self.groups = (checked, varied)
+
+        def unit_groups(self):
+            return self.groups
+
+    params = {"nsamps": 1 << 22}
+    one = (1 << 22) * 755
+    assert bench.fold_reads(params, Ffa(4, 0)) == one
+    assert bench.fold_reads(params, Ffa(4, 1)) == one * 5 // 4
+    assert bench.fold_reads(params, Ffa(4, 4)) == 2 * one
+    assert bench.fold_reads(params, Ffa(0, 0)) == 2 * one

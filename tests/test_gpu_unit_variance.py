@@ -1,6 +1,7 @@
 """Brute fold of series with unit variances (E alone, two segments a lane):
 all ones, ones but for one sample of one group, zero variances at the end, and
-batches whose lengths leave part of a group out, against the oracle bit for bit."""
+batches whose lengths leave part of a group out, against the oracle bit for bit;
+the executor's own count of the groups shows which way they were folded."""
 
 from __future__ import annotations
 
@@ -28,8 +29,28 @@ def test_unit_variances(cuda, nbins, kind):
         v[-1000:] = 0.0
     cfg = PulsarSearchConfig(n, tsamp, nbins, 1.0, np.array(lims), use_fourier=False, bseg_ffa=n // 16)
     op = lko.plan_create(lko.make_cfg(n, tsamp, nbins, 1.0, lims, bseg_ffa=n // 16))
-    got = FFACUDA(cfg).execute(e, v)
+    ffa = FFACUDA(cfg)
+    got = ffa.execute(e, v)
     np.testing.assert_array_equal(got.view(np.uint32), lko.ffa(op, e, v).view(np.uint32))
+    # 256 segments: four groups checked, one of them with another variance
+    assert int(op.nsegments[0]) == 256
+    assert ffa.unit_groups() == (4, 0 if kind == "ones" else 1)
+
+
+def test_one_wave_folds_both_rows(cuda):
+    """A fold whose blocks all run at once is not checked."""
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.ffa import FFACUDA
+
+    n, lims = 1 << 16, [[20.0, 22.0]]
+    cfg = PulsarSearchConfig(n, 64e-6, 32, 1.0, np.array(lims), use_fourier=False, score_widths=[1, 2])
+    op = lko.plan_create(lko.make_cfg(n, 64e-6, 32, 1.0, lims))
+    e, _ = series(n, 18)
+    v = np.ones(n, np.float32)
+    ffa = FFACUDA(cfg)
+    got = ffa.execute(e, v)
+    np.testing.assert_array_equal(got.view(np.uint32), lko.ffa(op, e, v).view(np.uint32))
+    assert ffa.unit_groups() == (0, 0)
 
 
 def test_batch_lengths(cuda):
@@ -48,5 +69,7 @@ def test_batch_lengths(cuda):
     ffa = FFACUDA(cfg, max_batch=3)
     ffa.set_batch_lengths(t.tensor(lengths, dtype=t.int64, device="cuda"))
     got = ffa.execute_batch(t.from_numpy(es).cuda(), t.from_numpy(vs).cuda()).cpu().numpy()
+    # 128 segments a series: the fourth group holds the ends of the shorter two
+    assert int(op.nsegments[0]) == 128 and ffa.unit_groups() == (6, 1)
     for k in range(3):
         np.testing.assert_array_equal(got[k].view(np.uint32), lko.ffa(op, es[k], vs[k]).view(np.uint32))
