@@ -351,10 +351,13 @@ def test_multi_series_slots_identical(cuda):
 # brute fold (groups of 8 segments) and their folds set to +0.0, so folds and
 # scores are bit-identical to folding the zeros. Lengths cover a full series,
 # a partial last segment, fewer valid segments than one group, one sample and
-# none. Shapes: two rows per warp in shared memory, with TMEM warps, and one
-# row per warp (which folds everything).
+# none. Shapes: the run form (the default) and, walking samples, two rows per
+# warp in shared memory, with TMEM warps, and one row per warp (which folds
+# everything).
 LEN_CASES = {
-    "accel_nb32_pk": (1 << 17, 1e-3, 32, ((-300.0, 300.0), (5.0, 8.0)), None),
+    "accel_nb32_run": (1 << 17, 1e-3, 32, ((-300.0, 300.0), (5.0, 8.0)), None),
+    "freq_nb128_run": (1 << 18, 64e-6, 128, ((20.0, 40.0),), None),
+    "accel_nb32_pk": (1 << 17, 1e-3, 32, ((-300.0, 300.0), (5.0, 8.0)), (2, 8, 0)),
     "accel_nb32_tmem": (1 << 17, 1e-3, 32, ((-300.0, 300.0), (5.0, 8.0)), (2, 6, 8)),
     "freq_nb128_tmem": (1 << 18, 64e-6, 128, ((20.0, 40.0),), (2, 4, 8)),
     "freq_nb128_rows1": (1 << 18, 64e-6, 128, ((20.0, 40.0),), (1, 8, 0)),
@@ -375,9 +378,12 @@ def test_batch_lengths_skip_padding(cuda, name):
     if shape is not None:
         rows, ws, tw = shape
         tu = skip.tuning
-        tu.update(bf_rows=rows, bf_warps=ws + tw, bf_tmem_warps=tw)
+        tu.update(bf_rows=rows, bf_warps=ws + tw, bf_stages=3, bf_tmem_warps=tw)
         skip.set_tuning(tu)
         plain.set_tuning(tu)
+    for f in (skip, plain):  # the form that the case is for
+        got = tuple(f.tuning[k] for k in ("bf_rows", "bf_warps", "bf_stages", "bf_tmem_warps"))
+        assert got == ((rows, ws + tw, 3, tw) if shape is not None else (2, got[1], 32, 0))
     es = np.zeros((nb, n), np.float32)
     vs = np.zeros((nb, n), np.float32)
     for k, L in enumerate(lengths):

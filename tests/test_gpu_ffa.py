@@ -65,6 +65,26 @@ def test_brute_fold_bit_exact(cuda, name):
     np.testing.assert_array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+# The forms that walk samples (other frequencies, saved launch shapes) on bins
+# that step by one a run: both row counts, bins in one byte and in two.
+@pytest.mark.parametrize("rows", [1, 2])
+@pytest.mark.parametrize("nbins", [16, 64, 100, 256, 300, 512])
+def test_walking_forms_bit_exact(cuda, nbins, rows):
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.ffa import FFACUDA
+
+    n, lims = 2**17, [[10.0, 20.0]]
+    cfg = PulsarSearchConfig(n, 64e-6, nbins, 1.0, np.array(lims), use_fourier=False, score_widths=[1, 2])
+    op = lko.plan_create(lko.make_cfg(n, 64e-6, nbins, 1.0, lims))
+    ts_e, ts_v = series(n, 15)
+    ffa = FFACUDA(cfg)
+    ffa.set_tuning(dict(bf_rows=rows, bf_warps=1 if nbins > 256 else 3, bf_stages=3))
+    assert (ffa.tuning["bf_rows"], ffa.tuning["bf_stages"], ffa.tuning["bf_tmem_warps"]) == (rows, 3, 0)
+    got = ffa.execute(ts_e, ts_v)
+    np.testing.assert_array_equal(got.view(np.uint32), lko.ffa(op, ts_e, ts_v).view(np.uint32))
+    assert ffa.status() == 0
+
+
 @pytest.mark.parametrize("seglen", [4, 16, 96, 160])
 def test_brute_fold_short_and_partial_segments(cuda, seglen):
     """Segment lengths that are not whole 64-sample stages or 32-sample words."""
