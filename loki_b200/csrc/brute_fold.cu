@@ -1189,9 +1189,6 @@ BruteFoldDevice::BruteFoldDevice(const std::vector<double>& freqs, uint64_t segm
                std::getenv("LOKI_B200_BF_STAGES") == nullptr) {
         configure(2, 0, run_form_stages());
     }
-    if (m_nseg % 8 == 0) {
-        m_groups.alloc((1 + m_max_batch + m_max_batch * m_nseg / 8) * sizeof(uint32_t));
-    }
     m_ready = true;
     prepare(m_use_runs, m_rows);
 }
@@ -1539,10 +1536,17 @@ void BruteFoldDevice::fold(float* d_fold, cudaStream_t s, const uint64_t* d_lens
 
 // Segment-group table of a batch whose series hold d_lens samples each (two
 // rows per warp and nseg a multiple of 8; otherwise every segment is folded).
+void BruteFoldDevice::reserve_groups() {
+    if (m_nseg % 8 == 0 && m_groups.ptr == nullptr) {
+        m_groups.alloc((1 + m_max_batch + m_max_batch * m_nseg / 8) * sizeof(uint32_t));
+    }
+}
+
 bool BruteFoldDevice::make_groups(const uint64_t* d_lens, uint64_t nbatch, cudaStream_t s) {
     if (d_lens == nullptr || m_rows != 2 || m_nseg % 8 != 0) {
         return false;
     }
+    reserve_groups();
     seg_groups_kernel<<<1, 256, 0, s>>>(d_lens, static_cast<uint32_t>(nbatch), static_cast<uint32_t>(m_nseg),
                                         m_seglen, m_groups.as<uint32_t>());
     LK_CUDA(cudaGetLastError());

@@ -887,8 +887,9 @@ void RunFold::reserve() {
     if (m_evt.ptr != nullptr) {
         return;
     }
-    m_varied.alloc((m_max_rows + 63) / 64 * sizeof(uint32_t));
-    m_evt.alloc(transposed_bytes(m_max_rows, m_nstages));
+    // the series, then the flags of the groups of 64
+    m_evt.alloc(transposed_bytes(m_max_rows, m_nstages) + (m_max_rows + 63) / 64 * sizeof(uint32_t));
+    m_varied = reinterpret_cast<uint32_t*>(m_evt.as<unsigned char>() + transposed_bytes(m_max_rows, m_nstages));
     // the zeros before and after each segment stay; the samples between them
     // are written by every call, on any stream
     LK_CUDA(cudaMemsetAsync(m_evt.ptr, 0, m_evt.bytes, nullptr));
@@ -906,22 +907,24 @@ void RunFold::transpose(const float* d_e, const float* d_v, uint64_t nrows, uint
     m_rows = nrows;
     const uint64_t g64 = (nrows + 63) / 64;
     if (m_unit) {
-        LK_CUDA(cudaMemsetAsync(m_varied.ptr, 0, g64 * sizeof(uint32_t), s));
+        LK_CUDA(cudaMemsetAsync(m_varied, 0, g64 * sizeof(uint32_t), s));
         pair_e_kernel<<<static_cast<unsigned>(g64 * tiles), 256, 0, s>>>(
             d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen, m_pad, static_cast<uint32_t>(qlen),
-            vec4, groups, ngroups, m_varied.as<uint32_t>());
+            vec4, groups, ngroups, m_varied);
         LK_CUDA(cudaGetLastError());
     }
     transpose_ev_kernel<<<static_cast<unsigned>(ngrp * tiles), 256, 0, s>>>(d_e, d_v, m_evt.as<float2>(), static_cast<uint32_t>(nrows), m_seglen,
                                              m_pad, static_cast<uint32_t>(qlen), vec4, groups, ngroups,
-                                             m_unit ? m_varied.as<uint32_t>() : nullptr);
+                                             m_unit ? m_varied : nullptr);
     LK_CUDA(cudaGetLastError());
 }
 
 void RunFold::unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const {
     std::vector<uint32_t> flags(m_unit ? (m_rows + 63) / 64 : 0);
-    LK_CUDA(cudaMemcpyAsync(flags.data(), m_varied.ptr, flags.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    LK_CUDA(cudaStreamSynchronize(s));
+    if (!flags.empty()) {
+        LK_CUDA(cudaMemcpyAsync(flags.data(), m_varied, flags.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        LK_CUDA(cudaStreamSynchronize(s));
+    }
     *checked = flags.size();
     *varied = static_cast<uint64_t>(std::count_if(flags.begin(), flags.end(), [](uint32_t x) { return x != 0; }));
 }
@@ -949,7 +952,7 @@ void RunFold::fold(float* d_fold, uint64_t nrows, uint32_t warps, const uint32_t
     a.status = d_status;
     a.groups = groups;
     a.ngroups = ngroups;
-    a.varied = m_unit ? m_varied.as<uint32_t>() : nullptr;
+    a.varied = m_unit ? m_varied : nullptr;
     a.counts = m_counts.as<float>();
     const uint64_t gy = static_cast<uint64_t>(a.nfb) * m_nranges;
     require(gy <= 65535, "BruteFold: too many frequencies for the launch grid");

@@ -316,6 +316,10 @@ int lk_ffa_search_batch(lk_ffa* ffa, const float* d_ts_e, const float* d_ts_v, u
 int lk_ffa_set_batch_lengths(lk_ffa* ffa, const uint64_t* d_lengths) {
     return guarded([&] {
         need(ffa, "ffa");
+        if (d_lengths != nullptr) {
+            lk::DeviceGuard g(ffa->exec->device);
+            ffa->exec->bf->reserve_groups();
+        }
         ffa->exec->batch_lens = d_lengths;
     });
 }

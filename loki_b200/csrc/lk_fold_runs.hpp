@@ -64,7 +64,7 @@ public:
     // (synchronises s).
     void unit_groups(uint64_t* checked, uint64_t* varied, cudaStream_t s) const;
     uint64_t device_bytes() const {
-        return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes + m_varied.bytes;
+        return m_items.bytes + m_rots.bytes + m_bits.bytes + m_counts.bytes + m_evt.bytes;
     }
 
 private:
@@ -76,7 +76,8 @@ private:
     uint32_t m_nranges = 1, m_range = 0;  // bin ranges per frequency, bins per range
     uint32_t m_pad = 0;                   // zero samples before each segment
     uint32_t m_nstages = 0;               // stages of one padded segment
-    DeviceBuffer m_items, m_rots, m_bits, m_counts, m_varied, m_evt;
+    DeviceBuffer m_items, m_rots, m_bits, m_counts, m_evt;
+    uint32_t* m_varied = nullptr;         // inside m_evt: flags of the groups of 64 segments
     uint32_t m_wpr = 1;
     uint64_t m_max_rows;
 };

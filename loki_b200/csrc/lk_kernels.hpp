@@ -81,6 +81,9 @@ public:
     uint32_t max_warps(uint32_t rows, uint32_t stages) const;
     // Most tensor-memory warps a block of smem_warps shared-memory warps can add.
     uint32_t max_tmem_warps(uint32_t smem_warps) const;
+    // Makes room for the segment-group table of max_batch series, which calls
+    // with d_lens use.
+    void reserve_groups();
     bool has_run_form() const;
     static uint32_t run_form_stages();
     uint32_t max_run_form_warps() const;

@@ -136,7 +136,7 @@ def test_ffa_fold_and_scores_bit_exact(cuda, name):
     assert ffa.status() == 0
 
 
-@pytest.mark.parametrize("name", ["freq_nb64", "accel_multi_nb32", "jerk_multi_nb32"])
+@pytest.mark.parametrize("name", ["freq_nb64", "freq_nb100_generic", "accel_multi_nb32", "jerk_multi_nb32"])
 def test_search_matches_ordered_compaction(cuda, name):
     from loki_b200.ffa import FFACUDA
 

@@ -133,6 +133,45 @@ def test_sweep_larger_chunked_vs_oracle(cuda):
         assert np.any(np.abs(params[:, 1] - f0) < 0.05 * f0)
 
 
+@pytest.mark.parametrize("executors,autotune", [("resident", False), ("resident", True), ("one_at_a_time", True)])
+def test_sweep_of_both_fold_forms(cuda, executors, autotune):
+    """Coarsely sampled data: the chunks of short segments fold by walking
+    samples, the others by runs, in one sweep."""
+    import ctypes
+
+    from loki_b200 import _capi as C
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.sweep import FFAFreqSweepCUDA
+    from oracle import lko
+
+    nsamps, tsamp = 1 << 17, 1e-3
+    lims = [[5.0, 200.0]]
+    ts_e, ts_v = series(nsamps, 78)
+    tt = np.arange(nsamps) * tsamp
+    for f0 in (6.1, 33.0, 121.0):
+        ts_e += (0.3 * (np.mod(tt * f0, 1.0) < 0.2)).astype(np.float32)
+    cfg = PulsarSearchConfig(nsamps, tsamp, 16, 1.0, np.array(lims), use_fourier=False,
+                             max_passing_candidates=1 << 16, snr_min=6.0)
+    sw = FFAFreqSweepCUDA(cfg, decode_chunk_widths=True, executors=executors, autotune=autotune)
+    rows = np.array([[c["f_min"], c["f_max"], c["nbins"], c["eta"]] for c in sw.chunks])
+    forms = set()
+    for f_min, f_max, nbins, eta in rows:
+        op = lko.plan_create(lko.make_cfg(nsamps, tsamp, int(nbins), eta, [[f_min, f_max]]))
+        f = op.freqs0()
+        form, size = ctypes.c_int(-1), ctypes.c_uint64()
+        C.check(C.lib().lk_brute_fold_form(f.ctypes.data, f.size, int(op.segment_lens[0]), int(nbins), nsamps, tsamp,
+                                           op.t_ref0(), 1, ctypes.byref(form), ctypes.byref(size)))
+        forms.add(form.value)
+    assert forms == {0, 1}
+    o_params, o_snr, o_counts = osweep.run((nsamps, tsamp, 16, 1.0, lims), rows, ts_e, ts_v, 6.0, chunk_widths=True)
+    for _ in range(2):
+        params, snr = sw.run(ts_e, ts_v)
+        np.testing.assert_array_equal(sw.region_counts, o_counts)
+        np.testing.assert_array_equal(params, o_params)
+        np.testing.assert_array_equal(snr.view(np.uint32), o_snr.view(np.uint32))
+    assert snr.size > 0
+
+
 def test_sweep_octaves_to_nbins_max_vs_oracle(cuda):
     """A plain period sweep over 1-250 Hz whose octaves grow from 62 to the
     1024-bin cap (the brute fold's widest accumulators, the generic merge and
