@@ -26,11 +26,14 @@
 // samples -- every frequency reads every sample once -- and 16 per run for its
 // sums, at 128 bytes per clock and SM. Measured on B200: the 2^22-sample
 // accelerated workload (nbins 64, 755 frequencies, 5-49 samples per run) 1.08
-// ms, 84 % of the shared-memory wavefront rate (1.83 ms walking samples, 1.56
+// ms, 83 % of the shared-memory wavefront rate (1.83 ms walking samples, 1.56
 // with its launch shape tuned and tensor-memory warps); the 2^21-sample period
 // sweep (nbins 128, 3020 frequencies) 3.23 against 6.91; nbins 100 0.41
 // against 0.74; 512 bins 0.86 against 3.18; 1024 bins 0.39 against 2.79; 64
-// segments of 50 frequencies (nbins 32) 0.023 against 0.056.
+// segments of 50 frequencies (nbins 32) 0.023 against 0.056. Series with unit
+// variances fold E alone (see pairs_e): 0.60 ms and 76 % of the wavefront rate at
+// 64 bins, 1.83 ms and 61 % at 128, where runs of 2 to 24 samples leave their
+// sums' 16 bytes and latency to weigh more.
 //
 // Keeping the sums in registers (the bin loop unrolled, a few runs' code per
 // bin) saves the 16 bytes but measured slower: the unrolled code outgrows the
