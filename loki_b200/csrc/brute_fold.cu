@@ -1,4 +1,6 @@
-// Brute fold (level 0 of the FFA) on sm_100a.
+// Brute fold (level 0 of the FFA) on sm_100a: the forms that walk samples, for
+// frequencies and segments that the run form (brute_fold_runs.cu, the default) does
+// not take and for saved launch shapes, and the choice between them.
 //
 // out[seg, f, r, b] = sum over samples i of segment seg whose phase bin at
 // frequency f is b, of ts_r[seg * seglen + i], added in increasing i starting
@@ -25,7 +27,7 @@
 //    run's bin by warp shuffle and reloads that bin's accumulators. All lanes
 //    follow the same mask, so control flow is uniform.
 //
-// Packed form (both rows per warp, the default for nbins <= 64): the series
+// Packed form (both rows per warp, the walking default for nbins <= 64): the series
 // is first interleaved into (e, v) pairs, so one 16-byte shared-memory load
 // yields two samples' pairs in adjacent registers and each sample is one
 // add.rn.f32x2 (two IEEE round-to-nearest adds, E and V, in one

@@ -457,8 +457,8 @@ lk_tuning FFAExec::autotune(const float* ts_e, const float* ts_v, uint32_t reps,
         // best packed (two-row) shared-memory shape, the base of step 1b
         float pk_best = INFINITY;
         uint32_t pw = 0, ps = stages0;
-        // The run form was faster than every shape of the other forms at each
-        // size tried, so where the plan has it only its warps are tuned.
+        // Where the plan has the run form it was faster than the other forms'
+        // shapes (see run_form_pays), so only its warps are tuned.
         const bool runs = bf->has_run_form();
         for (uint32_t w = runs ? bf->max_run_form_warps() : 0; w >= 4; --w) {
             if (!bf->configure(2, w, BruteFoldDevice::run_form_stages())) {

@@ -296,7 +296,8 @@ rfft_kernel(const float* __restrict__ in, float2* __restrict__ out, uint64_t npr
 // memory, in two steps of small transforms in registers (the direct sums above
 // take n operations a value and measured 8.96 / 7.84 ms on the 1.5 million
 // level-0 / final rows of the 2^21-sample period search at 128 bins, against
-// 0.39 / 0.44 here; what bounds these is the row traffic):
+// 0.39 / 0.44 here; shared memory bounds these, 77 / 63 % of the
+// wavefront rate with DRAM at 46 / 40 %, and the barriers between the steps):
 //   j = a B + b, m = a' + A b':
 //   Y[a'][b] = sum_a x[a B + b] e^{-2 pi i a a' / A}   (two columns b as one
 //              complex transform; a' <= A / 2, the rest are conjugates)

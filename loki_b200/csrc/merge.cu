@@ -199,9 +199,11 @@ __global__ void __launch_bounds__(kThreads)
 // registers from their own two parents (the same adds in the same tree, rounded
 // to BF16 where that level is stored so) instead of being written and read
 // back. Levels of hundreds of MB are bound by that traffic (a level's reads of
-// shared parents hit L1 and L2): 2 x 8 merge levels of the 2^21-sample period
-// search at 128 bins take 1.33 ms against 1.86, those of the 2^22-sample
-// accelerated search 0.28 against 0.33; small levels save a launch each.
+// shared parents hit L1 and L2): the seven merge levels of the 2^21-sample period
+// search at 128 bins take 1.32 ms in three pairs and one alone against 1.86, those
+// of the 2^22-sample accelerated search 0.25 against 0.33 (a pair of 25-Mfloat
+// levels 54 us and 156 MB of DRAM traffic against 2 x 39 us and 2 x 198 MB); small
+// levels save a launch each. Where a pair pays: pair_levels in ffa.cu.
 // NB: nbins, or 0 at run time. PB rows per warp and UJ times 32 bins of each in
 // flight, eight loads an element.
 template <bool TAYLOR, class TIn, class TOut, bool MID16, int NB, int PB, int UJ>
