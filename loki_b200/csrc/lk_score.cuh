@@ -393,9 +393,11 @@ inline uint32_t profiles_per_block(uint32_t rs) {
     return T;
 }
 
+// Raises the kernel's limit of dynamic shared memory where it is needed: above
+// 48 KB together with the kernel's static arrays (at most a few KB).
 template <class K>
 void set_smem(K kern, size_t smem) {
-    if (smem > 48 * 1024) {
+    if (smem > 40 * 1024) {
         LK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
     }

@@ -44,6 +44,22 @@ def test_mc_cascade_bit_exact(cuda):
     assert 0 < got[-1]["kept"] < got[0]["alive"]
 
 
+@pytest.mark.parametrize("nbins", [79, 111, 175, 367])
+def test_mc_rows_that_just_fit(cuda, nbins):
+    """Row lengths (bins + widest width) whose blocks take 48 KB of dynamic shared
+    memory less what the kernel's counters need on top."""
+    from loki_b200.synthetic import mc_cascade_workload
+    from loki_b200.thresholds import mc_cascade
+
+    folds0, signal, cls, noises, thresholds, grids = mc_cascade_workload(ntrials=3000, nbins=nbins, nstages=2, seed=6)
+    want = oracle_cascade(folds0, signal, cls, noises, thresholds, grids)
+    got = mc_cascade(folds0, signal, noises, cls, WIDTHS, thresholds, grids)
+    for g, w in zip(got, want):
+        assert (g["alive"], g["kept"]) == (w["alive"], w["kept"])
+        np.testing.assert_array_equal(g["counts"].astype(np.uint64), w["counts"])
+        np.testing.assert_array_equal(g["counts_flagged"].astype(np.uint64), w["counts_flagged"])
+
+
 @pytest.mark.parametrize("per_trial", [False, True])
 def test_mc_stage_folds_ids_and_max_snr(cuda, per_trial):
     from loki_b200.thresholds import MCStageCUDA
