@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(640, 1)
                 ring + static_cast<size_t>(s) * kStageBytes + row0 * kTileBytes + lrow;
             float x0[32];
             [[maybe_unused]] float x1[ROWS == 2 ? 32 : 1];
+            uint32_t z = 0;
 #pragma unroll
             for (uint32_t j = 0; j < 8; ++j) {
                 const uint32_t o = (j ^ lsw) << 4;
@@ -335,15 +336,18 @@ __global__ void __launch_bounds__(640, 1)
                 x0[4 * j + 1] = v0.y;
                 x0[4 * j + 2] = v0.z;
                 x0[4 * j + 3] = v0.w;
+                z ^= __float_as_uint(v0.x);
                 if constexpr (ROWS == 2) {
                     const float4 v1 = *reinterpret_cast<const float4*>(te + kTileBytes + o);
                     x1[4 * j + 0] = v1.x;
                     x1[4 * j + 1] = v1.y;
                     x1[4 * j + 2] = v1.z;
                     x1[4 * j + 3] = v1.w;
+                    z ^= __float_as_uint(v1.x);
                 }
             }
             // Release the stage as soon as its samples are in registers.
+            ptx::loads_done(z, &full[s], phase);
             ptx::mbar_arrive(&empty[s]);
             s = (s + 1 == S) ? 0 : s + 1;
             if (s == 0) {
@@ -576,6 +580,7 @@ __global__ void __launch_bounds__(640, 1)
             }
             const unsigned char* t0 = ring + static_cast<size_t>(s) * kStageBytes + lrow;
             float2 x[32];
+            uint32_t z = 0;
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
 #pragma unroll
@@ -584,8 +589,10 @@ __global__ void __launch_bounds__(640, 1)
                     const float4 v = *reinterpret_cast<const float4*>(t0 + h * kTileBytes + o);
                     x[16 * h + 2 * j] = make_float2(v.x, v.y);
                     x[16 * h + 2 * j + 1] = make_float2(v.z, v.w);
+                    z ^= __float_as_uint(v.x);
                 }
             }
+            ptx::loads_done(z, &full[s], phase);
             ptx::mbar_arrive(&empty[s]);
             s = (s + 1 == S) ? 0 : s + 1;
             if (s == 0) {
@@ -842,6 +849,7 @@ __global__ void __launch_bounds__(kMaxWarpsTm * 32, 1)
                 }
                 const unsigned char* t0 = ring + static_cast<size_t>(s) * kStageBytes + lrow;
                 uint32_t rl = static_cast<uint32_t>(r - rbase);
+                uint32_t z = 0;
                 // the word in two halves of 16 samples (fewer registers, so
                 // more warps fit)
 #pragma unroll
@@ -853,8 +861,10 @@ __global__ void __launch_bounds__(kMaxWarpsTm * 32, 1)
                         const float4 v = *reinterpret_cast<const float4*>(t0 + h * kTileBytes + o);
                         x[2 * j] = make_float2(v.x, v.y);
                         x[2 * j + 1] = make_float2(v.z, v.w);
+                        z ^= __float_as_uint(v.x);
                     }
                     if (h == 1) {
+                        ptx::loads_done(z, &full[s], phase);
                         ptx::mbar_arrive(&empty[s]);
                     }
                     const uint32_t mh = m >> (16 * h);

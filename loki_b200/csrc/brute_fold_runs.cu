@@ -139,8 +139,12 @@ struct Ring {
         gslot = gslot + 1 == a.slots ? 0 : gslot + 1;
     }
     // Waits until the samples below q_end have landed (false when a wait gave
-    // up); those below q are no longer needed by this warp.
-    __device__ __forceinline__ bool acquire(uint32_t q, uint32_t q_end, const RunArgs& a, int lane) {
+    // up); those below q are no longer needed by this warp. sum: one that the
+    // samples read last went into, where it has not been stored (a store needs
+    // its value, so the loads behind it are done).
+    __device__ __forceinline__ bool acquire(uint32_t q, uint32_t q_end, const RunArgs& a, int lane,
+                                            float sum = 0.0f) {
+        ptx::loads_done(__float_as_uint(sum), full_bar(a, hslot), hparity);
 #pragma unroll 1
         do {
 #pragma unroll 1
@@ -268,7 +272,7 @@ __device__ __forceinline__ bool fold_item(unsigned char* sums, Ring& rg, const R
                     float2 s = *reinterpret_cast<const float2*>(acc);
 #pragma unroll 1
                     for (uint32_t c = 0; c < nfull; ++c) {
-                        if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane)) {
+                        if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane, s.x)) {
                             return false;
                         }
                         s = add_run<kChunk - 1>(s, ring + off, true);
@@ -276,7 +280,7 @@ __device__ __forceinline__ bool fold_item(unsigned char* sums, Ring& rg, const R
                         off += kChunk * kSampleBytes;
                         off = off >= rbytes ? off - rbytes : off;
                     }
-                    if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane)) {
+                    if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane, s.x)) {
                         return false;
                     }
                     *reinterpret_cast<float2*>(acc) = add_run<LF>(s, ring + off, (m & 1u) != 0);

@@ -85,6 +85,38 @@ def test_walking_forms_bit_exact(cuda, nbins, rows):
     assert ffa.status() == 0
 
 
+# (nbins, rows, warps, tensor-memory warps): few warps, so that several blocks
+# share an SM, and whole blocks
+SHAPES = [(300, 1, 1, 0), (300, 2, 1, 0), (512, 1, 1, 0), (128, 1, 3, 0), (128, 1, 4, 0), (64, 1, 1, 0), (64, 2, 3, 0),
+          (64, 2, 12, 0), (64, 2, 1, 4), (128, 2, 2, 8)]
+
+
+@pytest.mark.parametrize("nbins, rows, warps, tmem", SHAPES)
+@pytest.mark.parametrize("stages", [2, 3])
+def test_walking_forms_repeat(cuda, nbins, rows, warps, tmem, stages):
+    """The same fold again and again: a stage of the sample ring must not be
+    refilled before every lane has read it."""
+    from loki_b200.configs import PulsarSearchConfig
+    from loki_b200.ffa import FFACUDA
+
+    t = cuda
+    n, lims = 2**17, [[10.0, 20.0]]
+    cfg = PulsarSearchConfig(n, 64e-6, nbins, 1.0, np.array(lims), use_fourier=False, score_widths=[1, 2])
+    op = lko.plan_create(lko.make_cfg(n, 64e-6, nbins, 1.0, lims))
+    e, v = (t.from_numpy(x).cuda() for x in series(n, 16))
+    ffa = FFACUDA(cfg)
+    want = ffa.execute(e, v)
+    np.testing.assert_array_equal(want.cpu().numpy().view(np.uint32),
+                                  lko.ffa(op, e.cpu().numpy(), v.cpu().numpy()).view(np.uint32))
+    ffa.set_tuning(dict(bf_rows=rows, bf_warps=warps + tmem, bf_stages=stages, bf_tmem_warps=tmem))
+    out = t.empty_like(want)
+    for _ in range(40):
+        out.zero_()
+        ffa.execute(e, v, out)
+        assert t.equal(out, want)
+    assert ffa.status() == 0
+
+
 @pytest.mark.parametrize("seglen", [4, 16, 96, 160])
 def test_brute_fold_short_and_partial_segments(cuda, seglen):
     """Segment lengths that are not whole 64-sample stages or 32-sample words."""
