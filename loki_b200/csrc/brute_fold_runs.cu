@@ -139,12 +139,10 @@ struct Ring {
         gslot = gslot + 1 == a.slots ? 0 : gslot + 1;
     }
     // Waits until the samples below q_end have landed (false when a wait gave
-    // up); those below q are no longer needed by this warp. sum: one that the
-    // samples read last went into, where it has not been stored (a store needs
-    // its value, so the loads behind it are done).
-    __device__ __forceinline__ bool acquire(uint32_t q, uint32_t q_end, const RunArgs& a, int lane,
-                                            float sum = 0.0f) {
-        ptx::loads_done(__float_as_uint(sum), full_bar(a, hslot), hparity);
+    // up); those below q are no longer needed by this warp: the loads of all of
+    // them are done, as their sums have been stored (an arrival alone does not
+    // wait for loads, see ptx::loads_done).
+    __device__ __forceinline__ bool acquire(uint32_t q, uint32_t q_end, const RunArgs& a, int lane) {
 #pragma unroll 1
         do {
 #pragma unroll 1
@@ -269,10 +267,13 @@ __device__ __forceinline__ bool fold_item(unsigned char* sums, Ring& rg, const R
                     q += adv;
                     off += adv * kSampleBytes;
                 } else {
+                    // (the chunk before is kept, its samples' sum is in a register and
+                    // the adds that used the one before that came first; q starts
+                    // kChunk or more into the padding)
                     float2 s = *reinterpret_cast<const float2*>(acc);
 #pragma unroll 1
                     for (uint32_t c = 0; c < nfull; ++c) {
-                        if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane, s.x)) {
+                        if (q + kChunk > rg.have && !rg.acquire(q - kChunk, q + kChunk, a, lane)) {
                             return false;
                         }
                         s = add_run<kChunk - 1>(s, ring + off, true);
@@ -280,7 +281,7 @@ __device__ __forceinline__ bool fold_item(unsigned char* sums, Ring& rg, const R
                         off += kChunk * kSampleBytes;
                         off = off >= rbytes ? off - rbytes : off;
                     }
-                    if (q + kChunk > rg.have && !rg.acquire(q, q + kChunk, a, lane, s.x)) {
+                    if (q + kChunk > rg.have && !rg.acquire(q - kChunk, q + kChunk, a, lane)) {
                         return false;
                     }
                     *reinterpret_cast<float2*>(acc) = add_run<LF>(s, ring + off, (m & 1u) != 0);
@@ -804,7 +805,7 @@ bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uin
                 const uint32_t upr = (it.bins + ub - 1) / ub;
                 const uint32_t uend = r + 1 < it.nrot ? upr : std::min(upr, it.t1 * (4 / ub));
                 for (uint32_t u = r == 0 ? it.t0 * (4 / ub) : 0; u < uend; ++u) {
-                    require(q >= released && q + (ub == 1 ? it.len + kChunk : ub * (it.len + 1)) <= qlen,
+                    require(q >= released && (ub > 1 || q >= kChunk) && q + (ub == 1 ? it.len + kChunk : ub * (it.len + 1)) <= qlen,
                             "run fold table: unit outside the segment");
                     released = q / kStageLen * kStageLen;
                     for (uint32_t b = u * ub; b < (u + 1) * ub; ++b) {

@@ -12,11 +12,11 @@
 
 namespace lk {
 
-// Host threads for n items of `each` units of work: one per 8192 units, about
-// 50 us of the table builders' arithmetic against 15 us for starting a thread,
+// Host threads for n items of `each` units of work: one per 32,768 units, about
+// 200 us of the table builders' work against up to as much for starting a thread,
 // at most 32.
 inline unsigned host_threads(uint64_t n, uint64_t each) {
-    const uint64_t want = n * (each + 1) / 8192 + 1;
+    const uint64_t want = n * (each + 1) / 32768 + 1;
     return static_cast<unsigned>(
         std::min<uint64_t>({want, std::max<uint64_t>(n, 1), 32, std::max(1u, std::thread::hardware_concurrency())}));
 }
