@@ -1274,6 +1274,9 @@ void BruteFoldDevice::make_tables() {
     LK_CUDA(cudaMemcpy(m_nruns.ptr, nruns.data(), m_nruns.bytes, cudaMemcpyHostToDevice));
     m_seq.alloc(m_nfreq);
     LK_CUDA(cudaMemcpy(m_seq.ptr, seq.data(), m_nfreq, cudaMemcpyHostToDevice));
+    // a copy from pageable memory may return before it has landed, and folds run
+    // on streams that do not wait for the default one
+    LK_CUDA(cudaStreamSynchronize(nullptr));
 }
 
 BruteFoldDevice::~BruteFoldDevice() = default;

@@ -805,7 +805,8 @@ bool run_fold_replay(const std::vector<double>& freqs, uint64_t segment_len, uin
                 const uint32_t upr = (it.bins + ub - 1) / ub;
                 const uint32_t uend = r + 1 < it.nrot ? upr : std::min(upr, it.t1 * (4 / ub));
                 for (uint32_t u = r == 0 ? it.t0 * (4 / ub) : 0; u < uend; ++u) {
-                    require(q >= released && (ub > 1 || q >= kChunk) && q + (ub == 1 ? it.len + kChunk : ub * (it.len + 1)) <= qlen,
+                    const uint64_t end = q + (ub == 1 ? it.len + kChunk : ub * (it.len + 1));
+                    require(q >= released && (ub > 1 || q >= kChunk) && end <= qlen,
                             "run fold table: unit outside the segment");
                     released = q / kStageLen * kStageLen;
                     for (uint32_t b = u * ub; b < (u + 1) * ub; ++b) {
@@ -899,7 +900,8 @@ void RunFold::reserve() {
     m_evt.alloc(transposed_bytes(m_max_rows, m_nstages) + (m_max_rows + 63) / 64 * sizeof(uint32_t));
     m_varied = reinterpret_cast<uint32_t*>(m_evt.as<unsigned char>() + transposed_bytes(m_max_rows, m_nstages));
     // the zeros before and after each segment stay; the samples between them
-    // are written by every call, on any stream
+    // are written by every call, on any stream (the tables' copies have landed
+    // after the wait too)
     LK_CUDA(cudaMemsetAsync(m_evt.ptr, 0, m_evt.bytes, nullptr));
     LK_CUDA(cudaStreamSynchronize(nullptr));
 }
